@@ -39,139 +39,170 @@ namespace fdsp {
 // ---------------------------------------------------------------------------
 // device helpers
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
+using ChanMeta = OutMeta;
+
+// Counter value (n mod R) of the sample at block-relative index w: one
+// multiply-high below 2^32 (Lemire, Kaser & Kurz, "Faster remainder by direct
+// computation", 2019).
+__device__ __forceinline__ uint32_t nco_counter(const ChanMeta& cm, int64_t w) {
+  const int64_t pv = (int64_t)cm.base + w;
+  if (pv < 0) return (uint32_t)(pv + (int64_t)cm.rollover);
+  if ((pv >> 32) == 0) return (uint32_t)__umul64hi(cm.fastmod * (uint64_t)(uint32_t)pv, (uint64_t)cm.rollover);
+  return (uint32_t)((uint64_t)pv % cm.rollover);
 }
 
-// (pv mod R) for 0 <= pv < 2^32 with a precomputed M = ceil(2^64 / R)
-// (Lemire, Kaser & Kurz, "Faster remainder by direct computation", 2019).
-__device__ __forceinline__ uint32_t fastmod_u32(uint32_t a, uint64_t M, uint32_t R) {
-  return (uint32_t)__umul64hi(M * (uint64_t)a, (uint64_t)R);
-}
-
-// Counter value (n mod R) of the sample at block-relative index w.
-__device__ __forceinline__ uint32_t nco_counter(const NcoConst& nc, uint32_t base, int64_t w) {
-  const int64_t pv = (int64_t)base + w;
-  if (pv < 0) return (uint32_t)(pv + (int64_t)nc.rollover);
-  if (pv < 0x100000000LL) return fastmod_u32((uint32_t)pv, nc.fastmod, nc.rollover);
-  return (uint32_t)((uint64_t)pv % nc.rollover);
-}
-
-// e^{j 2 pi t} for t in 2^-64 turns, on the SFU: the reduced argument lies in
+// e^{j 2 pi t} for t in 2^-32 turns, on the SFU: the reduced argument lies in
 // [-pi, pi), where __sincosf is accurate to ~4e-7 absolute.
-__device__ __forceinline__ float2 phasor64_fast(uint64_t turns64) {
-  const int32_t top = (int32_t)(turns64 >> 32);
-  const float a = (float)top * 1.4629180792671596e-09f;  // 2 pi / 2^32
+__device__ __forceinline__ float2 phasor32(uint32_t turns) {
+  const float a = (float)(int32_t)turns * 1.4629180792671596e-09f;  // 2 pi / 2^32
   float s, c;
   __sincosf(a, &s, &c);
   return make_float2(c, s);
 }
 
-using ChanMeta = OutMeta;
 
-// One row of one work set with NB live channels: T complex MACs per channel
-// (taps and samples from shared memory), then rotation and store.  Taps are
-// stored [T][NBS] with NBS = NB rounded up to even, so every row of taps
-// starts on a 16-byte boundary for the float4 loads.
-template <int NB>
-__device__ __forceinline__ void process_row(const float2* __restrict__ xs, const float2* __restrict__ tp,
-                                            const ChanMeta* __restrict__ meta, int T, int D, int P, int a0, int jl,
-                                            int64_t j, int U, int r, int delta) {
-  constexpr int NBS = (NB + 1) & ~1;  // tap row stride (even: 16-byte aligned rows)
-  int bq = a0 / D;
-  int b = a0 - bq * D;
-  const float2* xp = xs + b * P + bq + jl;
-  const int wrap = 1 - D * P;
-  // Narrow batches keep the two products of each complex MAC in separate
-  // accumulators so the FMA dependency chains stay short.
-  constexpr bool kSplit = NB <= 4;
-  float2 acc[NB], acc2[kSplit ? NB : 1];
+// Packed FP32 pairs: one instruction, two IEEE multiply-adds.  The FMA rate is
+// that of the scalar form (74 TFLOP/s of either measured); half the issue
+// slots stay free for the shared-memory reads.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+
+// kRows rows (jl, jl + 32, ...) of one work set with NB live channels: T
+// complex MACs per row and channel (taps and samples from shared memory), then
+// rotation and store.  Taps are stored [T][NB] as (re, re, im, im), so a
+// complex MAC is two packed multiply-adds of the sample as it lies in memory:
+// a += (re, re) x, b += (im, im) x, and the output is (a.x - b.y, a.y + b.x).
+// Bound: issue slots and shared-memory reads.  A tap read (a broadcast) feeds
+// kRows samples, a sample read NB channels.  Sums run over the taps in order
+// whatever kRows is, so an output's bits do not depend on the tile height.
+template <int NB, int kRows>
+__device__ __forceinline__ void process_rows(const float2* __restrict__ xs, const float4* __restrict__ tp,
+                                             const ChanMeta* __restrict__ meta, int T, int D, int P, int nph, int b0,
+                                             int q0, int64_t j, int64_t J, int U, int r, int delta) {
+  const f32x2* xp = reinterpret_cast<const f32x2*>(xs + b0 * P + q0);
+  const ulonglong2* tq = reinterpret_cast<const ulonglong2*>(tp);
+  const int wrap = 1 - nph * P;
+  f32x2 sa[kRows][NB], sb[kRows][NB];
 #pragma unroll
-  for (int n = 0; n < NB; ++n) acc[n] = make_float2(0.f, 0.f);
+  for (int q = 0; q < kRows; ++q)
 #pragma unroll
-  for (int n = 0; n < (kSplit ? NB : 1); ++n) acc2[n] = make_float2(0.f, 0.f);
+    for (int n = 0; n < NB; ++n) sa[q][n] = sb[q][n] = 0ull;
+  // runs of taps between the wraps of the de-interleaved tile
+  for (int k = 0, end = min(T, nph - b0); k < T; end = min(T, k + nph), xp += wrap) {
 #pragma unroll 2
-  for (int k = 0; k < T; ++k) {
-    const float2 x = *xp;
-    float2 gk[NB];
-    const float4* q4 = reinterpret_cast<const float4*>(tp + k * NBS);
+    for (; k < end; ++k) {
+      f32x2 x[kRows];
 #pragma unroll
-    for (int i = 0; i < NB / 2; ++i) {
-      const float4 v = q4[i];
-      gk[2 * i] = make_float2(v.x, v.y);
-      gk[2 * i + 1] = make_float2(v.z, v.w);
-    }
-    if constexpr (NB & 1) gk[NB - 1] = tp[k * NBS + NB - 1];
+      for (int q = 0; q < kRows; ++q) x[q] = xp[32 * q];
 #pragma unroll
-    for (int n = 0; n < NB; ++n) {
-      if constexpr (kSplit) {
-        acc[n].x = fmaf(gk[n].x, x.x, acc[n].x);
-        acc2[n].x = fmaf(-gk[n].y, x.y, acc2[n].x);
-        acc[n].y = fmaf(gk[n].x, x.y, acc[n].y);
-        acc2[n].y = fmaf(gk[n].y, x.x, acc2[n].y);
-      } else {
-        acc[n].x = fmaf(gk[n].x, x.x, acc[n].x);
-        acc[n].x = fmaf(-gk[n].y, x.y, acc[n].x);
-        acc[n].y = fmaf(gk[n].x, x.y, acc[n].y);
-        acc[n].y = fmaf(gk[n].y, x.x, acc[n].y);
+      for (int n = 0; n < NB; ++n) {
+        const ulonglong2 g = tq[n];
+#pragma unroll
+        for (int q = 0; q < kRows; ++q) {
+          sa[q][n] = fma2(g.x, x[q], sa[q][n]);
+          sb[q][n] = fma2(g.y, x[q], sb[q][n]);
+        }
       }
-    }
-    xp += P;
-    if (++b == D) {
-      b = 0;
-      xp += wrap;
+      xp += P;
+      tq += NB;
     }
   }
 
-  if constexpr (kSplit) {
+  float2 acc[kRows][NB];
+#pragma unroll
+  for (int q = 0; q < kRows; ++q)
 #pragma unroll
     for (int n = 0; n < NB; ++n) {
-      acc[n].x += acc2[n].x;
-      acc[n].y += acc2[n].y;
+      const float2 va = unpack2(sa[q][n]), vb = unpack2(sb[q][n]);
+      acc[q][n] = make_float2(va.x - vb.y, va.y + vb.x);
     }
-  }
 
-  // Epilogue: rotate by the NCO phase of the window start (branch free, so
-  // the channels' phase chains interleave), store; windows that straddle the
-  // NCO rollover take the exact split-sum path.
-  const int64_t m = (int64_t)r + (int64_t)U * j;
-  const int64_t w = (int64_t)delta + j * D - T + 1;  // window start, block relative
-  // The rare outputs that need the exact path (window across the NCO
-  // rollover) are first written unrotated, then fixed from that value, so no
-  // accumulator stays live through the fix-up.
-  uint32_t slow = 0;
+  // Epilogue: rotate by the NCO phase of the window start, store; windows that
+  // straddle the NCO rollover are stored unrotated and then take the exact
+  // split-sum path, so no accumulator stays live through the fix-up.  The
+  // counter of a channel's first row is one modulo, the next rows (32 D
+  // samples on) step it by 32 D mod R.
+  uint32_t slow = 0;  // bit q * NB + n
 #pragma unroll
   for (int n = 0; n < NB; ++n) {
-    float2 y = acc[n];
-    const bool ok = rotate_fast(meta[n], w, T, y);
-    meta[n].out[m] = ok ? y : acc[n];
-    slow |= ok ? 0u : (1u << n);
+    const ChanMeta& cm = meta[n];
+    const uint32_t R = cm.rollover, step = cm.step32;
+    const uint32_t om_lo = (uint32_t)cm.omega64, om_hi = (uint32_t)(cm.omega64 >> 32);
+    const bool en = cm.enabled != 0;
+    float2* const out = cm.out;
+    uint32_t p = en ? nco_counter(cm, (int64_t)delta + j * D - T + 1) : 0u;
+#pragma unroll
+    for (int q = 0; q < kRows; ++q) {
+      const float2 e0 = phasor32(__umulhi(p, om_lo) + p * om_hi);  // bits 32..63 of p * omega64
+      const float2 e = en ? e0 : make_float2(1.f, 0.f);
+      const bool ok = !en || (uint64_t)p + (uint64_t)T - 1 < (uint64_t)R;
+      const float2 y = cmul_nco(acc[q][n], e);
+      if (j + 32 * q < J) {
+        out[(int64_t)r + (int64_t)U * (j + 32 * q)] = ok ? y : acc[q][n];
+        slow |= ok ? 0u : (1u << (q * NB + n));
+      }
+      p += step;
+      p -= (p >= R || p < step) ? R : 0u;
+    }
   }
   while (slow) {
-    const int n = __ffs(slow) - 1;
+    const int bit = __ffs(slow) - 1;
     slow &= slow - 1;
+    const int q = bit / NB, n = bit - q * NB;
     const OutMeta& cm = meta[n];
-    const ExactRot er = rotate_prep(cm, w, T);
+    const int64_t jq = j + 32 * q;
+    const ExactRot er = rotate_prep(cm, (int64_t)delta + jq * D - T + 1, T);
     float2 B = make_float2(0.f, 0.f);
     if (er.straddle) {
-      const int kb = a0 + er.k0;
-      int qq = kb / D;
-      int bb = kb - qq * D;
-      qq += jl;
+      const int kb = b0 + er.k0;
+      int qq = kb / nph;
+      int bb = kb - qq * nph;
+      qq += q0 + 32 * q;
       for (int k = er.k0; k < T; ++k) {
         const float2 x = xs[bb * P + qq];
-        const float2 gk = tp[k * NBS + n];
+        const float4 g4 = tp[k * NB + n];
+        const float2 gk = make_float2(g4.x, g4.z);
         B.x = fmaf(gk.x, x.x, B.x);
         B.x = fmaf(-gk.y, x.y, B.x);
         B.y = fmaf(gk.x, x.y, B.y);
         B.y = fmaf(gk.y, x.x, B.y);
-        if (++bb == D) {
+        if (++bb == nph) {
           bb = 0;
           ++qq;
         }
       }
     }
-    cm.out[m] = rotate_apply(er, cm.out[m], B);
+    float2* o = cm.out + ((int64_t)r + (int64_t)U * jq);
+    *o = rotate_apply(er, *o, B);
+  }
+}
+
+// The row blocks of one work set: two rows a thread where the tile height
+// allows (four in engines of one or two channels a batch), one otherwise.
+template <int NB>
+__device__ __forceinline__ void process_block(int rows, const float2* __restrict__ xs, const float4* __restrict__ tp,
+                                              const ChanMeta* __restrict__ meta, int T, int D, int P, int nph, int b0,
+                                              int q0, int64_t j, int64_t J, int U, int r, int delta) {
+  if (NB <= 2 && rows == 4) {
+    process_rows<NB, NB <= 2 ? 4 : 2>(xs, tp, meta, T, D, P, nph, b0, q0, j, J, U, r, delta);
+  } else if (rows >= 2) {
+    process_rows<NB, 2>(xs, tp, meta, T, D, P, nph, b0, q0, j, J, U, r, delta);
+  } else {
+    process_rows<NB, 1>(xs, tp, meta, T, D, P, nph, b0, q0, j, J, U, r, delta);
   }
 }
 
@@ -186,23 +217,13 @@ __device__ __forceinline__ void process_row(const float2* __restrict__ xs, const
 // semantics) take 2 FMAs per tap instead of 4.
 constexpr int kWinRows = 7;
 
-template <bool kReal>
-__device__ __forceinline__ void win_mac(float2& acc, float2 g, float2 x) {
-  if constexpr (kReal) {
-    acc.x = fmaf(g.x, x.x, acc.x);
-    acc.y = fmaf(g.x, x.y, acc.y);
-  } else {
-    acc.x = fmaf(g.x, x.x, acc.x);
-    acc.x = fmaf(-g.y, x.y, acc.x);
-    acc.y = fmaf(g.x, x.y, acc.y);
-    acc.y = fmaf(g.y, x.x, acc.y);
-  }
-}
+// Shared memory of a CTA that leaves room for two more on the SM.
+constexpr int kSmem3 = 75 * 1024;
 
 // Rotation and store of one single-channel output (the per-row epilogue
-// for NB = 1, taps at stride 2 float2).
+// for NB = 1).
 __device__ __forceinline__ void win_finish(float2 acc, const ChanMeta& cm, const float2* __restrict__ xs,
-                                           const float2* __restrict__ tp, int T, int D, int P, int a0, int jl,
+                                           const float4* __restrict__ tp, int T, int D, int P, int a0, int jl,
                                            int64_t j, int U, int r, int delta) {
   const int64_t m = (int64_t)r + (int64_t)U * j;
   const int64_t w = (int64_t)delta + j * D - T + 1;
@@ -220,7 +241,8 @@ __device__ __forceinline__ void win_finish(float2 acc, const ChanMeta& cm, const
     qq += jl;
     for (int k = er.k0; k < T; ++k) {
       const float2 x = xs[bb * P + qq];
-      const float2 gk = tp[k * 2];
+      const float4 g4 = tp[k];
+      const float2 gk = make_float2(g4.x, g4.z);
       B.x = fmaf(gk.x, x.x, B.x);
       B.x = fmaf(-gk.y, x.y, B.x);
       B.y = fmaf(gk.x, x.y, B.y);
@@ -235,12 +257,14 @@ __device__ __forceinline__ void win_finish(float2 acc, const ChanMeta& cm, const
 }
 
 template <bool kReal>
-__device__ __forceinline__ void process_rows_win(const float2* __restrict__ xs, const float2* __restrict__ tp,
+__device__ __forceinline__ void process_rows_win(const float2* __restrict__ xs, const float4* __restrict__ tp,
                                                  const ChanMeta* __restrict__ meta, int T, int D, int P, int a0,
                                                  int jl0, int64_t j0, int64_t J, int U, int r, int delta) {
-  float2 acc[kWinRows];
+  // packed multiply-adds in the scalar form's order: (re, re) (x, y), then
+  // (-im, im) (y, x) for complex taps
+  f32x2 acc[kWinRows];
 #pragma unroll
-  for (int q = 0; q < kWinRows; ++q) acc[q] = make_float2(0.f, 0.f);
+  for (int q = 0; q < kWinRows; ++q) acc[q] = 0ull;
   const int bq = a0 / D, b0 = a0 - bq * D;
   const int nv = T < D ? T : D;
   for (int vp = 0; vp < nv; ++vp) {
@@ -249,108 +273,214 @@ __device__ __forceinline__ void process_rows_win(const float2* __restrict__ xs, 
       ph -= D;
       ++q0;
     }
-    const float2* xr = xs + ph * P + q0;  // row jl0 + q, tap vp + m D: xr[m + q]
-    const float2* tk = tp + 2 * vp;       // tap k at tp[2 k]
-    const int tstep = 2 * D;
+    const f32x2* xr = reinterpret_cast<const f32x2*>(xs + ph * P + q0);  // row jl0 + q, tap vp + m D: xr[m + q]
+    const ulonglong2* tk = reinterpret_cast<const ulonglong2*>(tp + vp);
     const int nm = (T - 1 - vp) / D + 1;
-    float2 w[kWinRows];
+    f32x2 w[kWinRows], sw[kReal ? 1 : kWinRows];  // samples, and with re and im exchanged
+    auto put = [&](int i, f32x2 v) {
+      w[i] = v;
+      if constexpr (!kReal) {
+        const float2 f = unpack2(v);
+        sw[i] = pack2(f.y, f.x);
+      }
+    };
+    auto tap = [&](int m, f32x2& gr, f32x2& gi) {
+      if constexpr (kReal) {
+        gr = tk[m * D].x;
+      } else {
+        const ulonglong2 g = tk[m * D];
+        const float2 f = unpack2(g.y);
+        gr = g.x;
+        gi = pack2(-f.x, f.y);
+      }
+    };
 #pragma unroll
-    for (int q = 0; q < kWinRows - 1; ++q) w[q] = xr[q];
+    for (int q = 0; q < kWinRows - 1; ++q) put(q, xr[q]);
     int m = 0;
     for (; m + kWinRows <= nm; m += kWinRows) {
       // circular window: sample m + u + q sits in slot (u + q) % kWinRows
 #pragma unroll
       for (int u = 0; u < kWinRows; ++u) {
-        w[(u + kWinRows - 1) % kWinRows] = xr[m + u + kWinRows - 1];
-        const float2 g = tk[(m + u) * tstep];
+        put((u + kWinRows - 1) % kWinRows, xr[m + u + kWinRows - 1]);
+        f32x2 gr, gi = 0ull;
+        tap(m + u, gr, gi);
 #pragma unroll
-        for (int q = 0; q < kWinRows; ++q) win_mac<kReal>(acc[q], g, w[(u + q) % kWinRows]);
+        for (int q = 0; q < kWinRows; ++q) {
+          acc[q] = fma2(gr, w[(u + q) % kWinRows], acc[q]);
+          if constexpr (!kReal) acc[q] = fma2(gi, sw[(u + q) % kWinRows], acc[q]);
+        }
       }
     }
     for (; m < nm; ++m) {
-      w[kWinRows - 1] = xr[m + kWinRows - 1];
-      const float2 g = tk[m * tstep];
+      put(kWinRows - 1, xr[m + kWinRows - 1]);
+      f32x2 gr, gi = 0ull;
+      tap(m, gr, gi);
 #pragma unroll
-      for (int q = 0; q < kWinRows; ++q) win_mac<kReal>(acc[q], g, w[q]);
+      for (int q = 0; q < kWinRows; ++q) {
+        acc[q] = fma2(gr, w[q], acc[q]);
+        if constexpr (!kReal) acc[q] = fma2(gi, sw[q], acc[q]);
+      }
 #pragma unroll
-      for (int q = 0; q < kWinRows - 1; ++q) w[q] = w[q + 1];
+      for (int q = 0; q < kWinRows - 1; ++q) {
+        w[q] = w[q + 1];
+        if constexpr (!kReal) sw[q] = sw[q + 1];
+      }
     }
   }
 #pragma unroll
   for (int q = 0; q < kWinRows; ++q)
-    if (j0 + q < J) win_finish(acc[q], meta[0], xs, tp, T, D, P, a0, jl0 + q, j0 + q, U, r, delta);
+    if (j0 + q < J) win_finish(unpack2(acc[q]), meta[0], xs, tp, T, D, P, a0, jl0 + q, j0 + q, U, r, delta);
 }
 
-// One CTA = one tile of Qt output rows of decimation group g.  Shared memory:
-// [input tile, de-interleaved: D x P float2][taps of every work set of the
-// group, packed [T][nb]][ChanMeta per (work set, channel)].
+// History after a block: the last H samples of [old history | block], sample
+// i of the new buffer.
+__device__ __forceinline__ void hist_sample(const float2* __restrict__ old_hist, const float2* __restrict__ block,
+                                            const short2* __restrict__ block16, int64_t N, int H,
+                                            float2* __restrict__ new_hist, int i) {
+  const int64_t v = N + i;
+  if (v < H) {
+    new_hist[i] = old_hist[v];
+  } else if (block16 != nullptr) {
+    const short2 s = block16[v - H];
+    new_hist[i] = make_float2((float)s.x, (float)s.y);
+  } else {
+    new_hist[i] = block[v - H];
+  }
+}
+
+// One CTA = one tile of Qt output rows of a decimation group; the tiles of the
+// launch's groups (fuse_map[first ..]) follow one another in blockIdx.x, and
+// the blocks past the last tile write the history of the next block.  Shared
+// memory: [input tile, de-interleaved: nph x P float2][taps of every work set
+// of the group, packed [T][nb]][ChanMeta per (work set, channel)].
+//
+// One launch over all groups: a group alone has 100-400 tiles, 1-2 a SM, so
+// launches one after another each ended in a nearly empty wave (64 channels of
+// 2^20 samples: 12 launches 165 us, one launch 82 us).
+//
+// The tile holds the input phases that some window reads: all D of them where
+// windows overlap or wrap, else (long decimations) only the groups' windows,
+// up to kMaxSegs segments of them (seg_at / seg_gap map a staged phase to its
+// place in the row).
 template <int NBMAX, bool kTapsSmem, bool kWin>
-__global__ void __launch_bounds__(kThreads, 3) poly_fp32_kernel(const __grid_constant__ PolyLaunch<NBMAX> L, int g) {
+__global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
+    poly_fp32_kernel(const __grid_constant__ PolyLaunch<NBMAX> L, int first, int tiles) {
   extern __shared__ __align__(16) float2 xs[];
-  // g < 0: one launch over several groups (small blocks), group =
-  // fuse_map[blockIdx.y + (-g - 1)]
-  const GroupDesc& G = L.groups[g >= 0 ? g : (int)L.fuse_map[(int)blockIdx.y - g - 1]];
-  const int tile = blockIdx.x;
-  if (tile >= G.ntiles) return;  // uniform over the CTA, before any barrier
-  const int D = G.D, Qt = G.Qt, P = G.P;
+  int tile = blockIdx.x;
+  if (tile >= tiles) {
+    const int i = (tile - tiles) * kThreads + (int)threadIdx.x;
+    if (i < L.H) hist_sample(L.hist, L.block, L.block16, L.N, L.H, L.new_hist, i);
+    return;
+  }
+  for (; tile >= L.groups[L.fuse_map[first]].ntiles; ++first) tile -= L.groups[L.fuse_map[first]].ntiles;
+  const GroupDesc& G = L.groups[L.fuse_map[first]];
+  const int D = G.D, Qt = G.Qt, P = G.P, nph = G.nph;
   const int64_t row0 = (int64_t)tile * Qt;
-  const int64_t sb = row0 * D + G.delta_min - G.tmax + 1;  // first staged input (block relative)
-  const int len = Qt * D + G.delta_span + G.tmax - 1;
-  float2* taps_s = xs + G.taps_off;
+  const int64_t sb = row0 * D + G.delta_min - G.tmax + 1 + G.seg_first;  // first staged input (block relative)
+  const int len = G.len;
+  float4* taps_s = reinterpret_cast<float4*>(xs + G.taps_off);
   ChanMeta* meta_s = reinterpret_cast<ChanMeta*>(xs + G.meta_off);
   const int nws = G.ws_end - G.ws_begin;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   // Stage the raw input span, de-interleaved by D, with asynchronous 8-byte
   // copies (every copy of the tile in flight at once).  Negative indices come
   // from the history (the H samples before the block); past the block end the
   // copy reads 0 bytes and zero-fills.
-  if (L.block16 == nullptr) {
-    for (int t = threadIdx.x; t < len; t += blockDim.x) {
-      const int64_t v = sb + t;
-      const float2* src = L.block;
-      uint32_t bytes = 0;
-      if (v < 0) {
-        const int64_t hv = v + L.H;
-        if (hv >= 0) {
-          src = L.hist + hv;
+  // Sample t of the tile is phase b = t mod nph of row q = t / nph, stepped
+  // by kThreads; a tile inside the block skips the range checks.
+  {
+    int q = (int)(((uint64_t)threadIdx.x * G.inv_nph) >> 32);
+    int b = (int)threadIdx.x - q * nph;
+    const int dq = G.step_q, db = G.step_b;
+    const int at0 = G.seg_at[0], at1 = G.seg_at[1], at2 = G.seg_at[2];
+    const int gap0 = G.seg_gap[0], gap1 = G.seg_gap[1], gap2 = G.seg_gap[2];
+    const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(xs);
+    auto place = [&]() {  // sample of the tile's span
+      return q * D + b + (b >= at0 ? gap0 : 0) + (b >= at1 ? gap1 : 0) + (b >= at2 ? gap2 : 0);
+    };
+    auto advance = [&]() {
+      b += db;
+      q += dq;
+      if (b >= nph) {
+        b -= nph;
+        ++q;
+      }
+    };
+    if (L.block16 == nullptr && sb >= 0 && sb + G.span <= L.N) {
+      const float2* src = L.block + sb;
+      if (nph == D) {
+        src += threadIdx.x;
+        for (int t = threadIdx.x; t < len; t += kThreads, src += kThreads, advance())
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst0 + 8u * (uint32_t)(b * P + q)), "l"(src)
+                       : "memory");
+      } else {
+        for (int t = threadIdx.x; t < len; t += kThreads, advance())
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst0 + 8u * (uint32_t)(b * P + q)),
+                       "l"(src + place())
+                       : "memory");
+      }
+    } else if (L.block16 == nullptr) {
+      for (int t = threadIdx.x; t < len; t += kThreads, advance()) {
+        const int64_t v = sb + place();
+        const float2* src = L.block;
+        uint32_t bytes = 0;
+        if (v < 0) {
+          const int64_t hv = v + L.H;
+          if (hv >= 0) {
+            src = L.hist + hv;
+            bytes = 8;
+          }
+        } else if (v < L.N) {
+          src = L.block + v;
           bytes = 8;
         }
-      } else if (v < L.N) {
-        src = L.block + v;
-        bytes = 8;
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst0 + 8u * (uint32_t)(b * P + q)),
+                     "l"(src), "r"(bytes)
+                     : "memory");
       }
-      const int q = t / D;
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(xs + (t - q * D) * P + q);
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-    }
-  } else {
-    // int16 front end: block samples are converted on the way in (the
-    // history is already float)
-    for (int t = threadIdx.x; t < len; t += blockDim.x) {
-      const int64_t v = sb + t;
-      const int q = t / D;
-      float2 x = make_float2(0.f, 0.f);
-      if (v < 0) {
-        const int64_t hv = v + L.H;
-        if (hv >= 0) x = L.hist[hv];
-      } else if (v < L.N) {
-        const short2 s = L.block16[v];
-        x = make_float2((float)s.x, (float)s.y);
+    } else {
+      // int16 front end: block samples are converted on the way in (the
+      // history is already float), four loads in flight a thread
+      for (int t = threadIdx.x; t < len;) {
+        float2 x[4];
+        int at[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u, t += kThreads, advance()) {
+          at[u] = -1;
+          x[u] = make_float2(0.f, 0.f);
+          if (t >= len) continue;
+          at[u] = b * P + q;
+          const int64_t v = sb + place();
+          if (v < 0) {
+            const int64_t hv = v + L.H;
+            if (hv >= 0) x[u] = L.hist[hv];
+          } else if (v < L.N) {
+            const short2 s = L.block16[v];
+            x[u] = make_float2((float)s.x, (float)s.y);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (at[u] >= 0) xs[at[u]] = x[u];
       }
-      xs[(t - q * D) * P + q] = x;
     }
   }
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
   // Stage the taps of every work set (when they fit) and the per-channel NCO
-  // constants.
-  for (int wi = 0; wi < nws; ++wi) {
+  // constants: a warp a work set, every copy in flight at once (one work set
+  // after another with plain loads took a memory latency each).
+  for (int wi = warp; wi < nws; wi += kThreads / 32) {
     const WorkSet<NBMAX>& W = L.ws[G.ws_begin + wi];
     if constexpr (kTapsSmem) {
-      const int cnt = W.T * ((W.nb + 1) & ~1);
-      for (int i = threadIdx.x; i < cnt; i += blockDim.x) taps_s[W.soff + i] = __ldg(W.taps + i);
+      const int cnt = W.T * W.nb;
+      const float4* src = W.taps;
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(taps_s + W.soff);
+      for (int i = lane; i < cnt; i += 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16u * (uint32_t)i), "l"(src + i)
+                     : "memory");
     }
-    if (threadIdx.x < W.nb) {
-      const int c = W.ch[threadIdx.x];
+    if (lane < W.nb) {
+      const int c = W.ch[lane];
       const NcoConst nc = L.nco[c];
       ChanMeta m;
       m.omega64 = nc.omega64;
@@ -360,10 +490,11 @@ __global__ void __launch_bounds__(kThreads, 3) poly_fp32_kernel(const __grid_con
       m.rollover = nc.rollover;
       m.base = L.nco_base[c];
       m.enabled = nc.enabled;
-      m.pad_ = 0;
-      meta_s[wi * NBMAX + threadIdx.x] = m;
+      m.step32 = nc.rollover ? (32u * (uint32_t)D) % nc.rollover : 0u;
+      meta_s[wi * NBMAX + lane] = m;
     }
   }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
 
@@ -380,7 +511,7 @@ __global__ void __launch_bounds__(kThreads, 3) poly_fp32_kernel(const __grid_con
       if (j0 >= W.J) continue;
       const int T = W.T;
       const int a0 = (W.delta - G.delta_min) + (G.tmax - T);
-      const float2* tp = kTapsSmem ? taps_s + W.soff : W.taps;
+      const float4* tp = kTapsSmem ? taps_s + W.soff : W.taps;
       const ChanMeta* mt = meta_s + wq * NBMAX;
       if (G.real_taps)
         process_rows_win<true>(xs, tp, mt, T, D, P, a0, jl0, j0, W.J, W.U, W.r, W.delta);
@@ -390,46 +521,45 @@ __global__ void __launch_bounds__(kThreads, 3) poly_fp32_kernel(const __grid_con
     return;
   }
 
-  // Items are (work set, row) with rows fastest; Qt is a multiple of 32 so a
-  // warp never mixes work sets and every tap load is a broadcast.
-  const int nitems = nws * Qt;
-  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    const int wq = it / Qt;
-    const int jl = it - wq * Qt;
+  // Items are (work set, block of 32 kRows rows), a warp each, so every tap
+  // load is a broadcast.
+  const int rows = G.rows;
+  const int nblk = Qt / (32 * rows);
+  const int nitems = nws * nblk;
+  for (int it = warp; it < nitems; it += kThreads / 32) {
+    const int wq = it / nblk;
+    const int jl = (it - wq * nblk) * 32 * rows;
     const WorkSet<NBMAX>& W = L.ws[G.ws_begin + wq];
-    const int64_t j = row0 + jl;
-    if (j >= W.J) continue;
-    const int T = W.T;
-    const int a0 = (W.delta - G.delta_min) + (G.tmax - T);
-    const float2* tp = kTapsSmem ? taps_s + W.soff : W.taps;
+    if (row0 + jl >= W.J) continue;
+    const int64_t j = row0 + jl + lane;
+    const int T = W.T, b0 = W.b0, q0 = W.q0 + jl + lane;
+    const float4* tp = kTapsSmem ? taps_s + W.soff : W.taps;
     const ChanMeta* mt = meta_s + wq * NBMAX;
+#define FDSP_NB(n)                                                                                        \
+  case n:                                                                                                 \
+    if constexpr (NBMAX >= n)                                                                             \
+      process_block<n>(rows, xs, tp, mt, T, D, P, nph, b0, q0, j, (int64_t)W.J, W.U, W.r, W.delta);       \
+    break;
     switch (W.nb) {
-      case 1: process_row<1>(xs, tp, mt, T, D, P, a0, jl, j, W.U, W.r, W.delta); break;
-      case 2: if constexpr (NBMAX >= 2) process_row<2>(xs, tp, mt, T, D, P, a0, jl, j, W.U, W.r, W.delta); break;
-      case 3: if constexpr (NBMAX >= 3) process_row<3>(xs, tp, mt, T, D, P, a0, jl, j, W.U, W.r, W.delta); break;
-      case 4: if constexpr (NBMAX >= 4) process_row<4>(xs, tp, mt, T, D, P, a0, jl, j, W.U, W.r, W.delta); break;
-      case 5: if constexpr (NBMAX >= 5) process_row<5>(xs, tp, mt, T, D, P, a0, jl, j, W.U, W.r, W.delta); break;
-      case 6: if constexpr (NBMAX >= 6) process_row<6>(xs, tp, mt, T, D, P, a0, jl, j, W.U, W.r, W.delta); break;
-      case 7: if constexpr (NBMAX >= 7) process_row<7>(xs, tp, mt, T, D, P, a0, jl, j, W.U, W.r, W.delta); break;
-      default: if constexpr (NBMAX >= 8) process_row<NBMAX>(xs, tp, mt, T, D, P, a0, jl, j, W.U, W.r, W.delta); break;
+      FDSP_NB(1)
+      FDSP_NB(2)
+      FDSP_NB(3)
+      FDSP_NB(4)
+      FDSP_NB(5)
+      FDSP_NB(6)
+      FDSP_NB(7)
+      FDSP_NB(8)
+      default: break;
     }
+#undef FDSP_NB
   }
 }
 
-// History after a block: the last H samples of [old history | block].
+// The history update alone (applies whose groups all ran on the tensor cores).
 __global__ void hist_update_kernel(const float2* __restrict__ old_hist, const float2* __restrict__ block,
                                    const short2* __restrict__ block16, int64_t N, int H, float2* __restrict__ new_hist) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= H) return;
-  const int64_t v = N + i;
-  if (v < H) {
-    new_hist[i] = old_hist[v];
-  } else if (block16 != nullptr) {
-    const short2 s = block16[v - H];
-    new_hist[i] = make_float2((float)s.x, (float)s.y);
-  } else {
-    new_hist[i] = block[v - H];
-  }
+  if (i < H) hist_sample(old_hist, block, block16, N, H, new_hist, i);
 }
 
 // ---------------------------------------------------------------------------
@@ -516,10 +646,12 @@ void DevPool::release(void* p) {
 }
 
 static int choose_qt(uint32_t D, int tmax) {
-  // ~4K input samples per tile (three CTAs per SM), at least one warp of rows,
-  // shared memory (tile + halo + offset spread, de-interleaved) under ~200 KB.
-  int qt = (int)((4096 / D) & ~31u);
-  if (qt < 32) qt = 32;
+  // ~4K input samples per tile (three CTAs per SM), two warps' rows where that
+  // stays within ~8K samples (a thread then computes two rows or more), at
+  // least one; shared memory (tile + halo + offset spread, de-interleaved)
+  // under ~200 KB.
+  int qt = (int)((4096 / D) & ~63u);
+  if (qt < 64) qt = D <= 128 ? 64 : 32;
   auto bytes = [&](int q) {
     const int64_t len = (int64_t)q * D + 3LL * D + tmax;
     const int64_t P = len / D + 2;
@@ -656,11 +788,11 @@ int PolyEngine::init(uint32_t fs, const fdsp_channel_cfg* ch, uint32_t nch, bool
     }
   }
 
-  // modulated, padded taps of every batch: [up][T][NB]
+  // modulated, padded taps of every batch: [up][T][channels] as (re, re, im, im)
   for (auto& bt : batches_) {
     const uint32_t U = classes_[bt.cls].up;
-    const size_t nb = (bt.chans.size() + 1) & ~(size_t)1;  // tap rows padded to an even width
-    std::vector<float2> host((size_t)U * bt.T * nb, make_float2(0.f, 0.f));
+    const size_t nb = bt.chans.size();
+    std::vector<float4> host((size_t)U * bt.T * nb, make_float4(0.f, 0.f, 0.f, 0.f));
     for (size_t n = 0; n < bt.chans.size(); ++n) {
       const EngineChannel& e = chans_[bt.chans[n]];
       const int pad = bt.T - (int)e.T;
@@ -681,13 +813,13 @@ int PolyEngine::init(uint32_t fs, const fdsp_channel_cfg* ch, uint32_t nch, bool
             gr = (double)h.x * c - (double)h.y * s;
             gi = (double)h.x * s + (double)h.y * c;
           }
-          host[((size_t)ph * bt.T + k) * nb + n] = make_float2((float)gr, (float)gi);
+          host[((size_t)ph * bt.T + k) * nb + n] = make_float4((float)gr, (float)gr, (float)gi, (float)gi);
         }
       }
     }
-    cudaError_t e = dalloc(reinterpret_cast<void**>(&bt.d_taps), host.size() * sizeof(float2));
+    cudaError_t e = dalloc(reinterpret_cast<void**>(&bt.d_taps), host.size() * sizeof(float4));
     if (e != cudaSuccess) return cuda_status(e);
-    e = cudaMemcpy(bt.d_taps, host.data(), host.size() * sizeof(float2), cudaMemcpyHostToDevice);
+    e = cudaMemcpy(bt.d_taps, host.data(), host.size() * sizeof(float4), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_status(e);
   }
 
@@ -898,6 +1030,103 @@ void PolyEngine::reset() {
   cudaDeviceSynchronize();
 }
 
+// Tile of Qt rows of one group: which input phases it stages, its pitch, and
+// its shared-memory layout.
+template <int NB>
+static void layout_group(PolyLaunch<NB>& L, GroupDesc& gd, int Qt) {
+  const int D = gd.D;
+  gd.Qt = Qt;
+  gd.rows = NB <= 2 && Qt % 128 == 0 ? 4 : Qt % 64 == 0 ? 2 : 1;
+  gd.nph = D;
+  for (int i = 0; i < kMaxSegs - 1; ++i) {
+    gd.seg_at[i] = INT32_MAX;
+    gd.seg_gap[i] = 0;
+  }
+  int64_t len = (int64_t)Qt * D + gd.delta_span + gd.tmax - 1;
+  for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) {
+    WorkSet<NB>& W = L.ws[wi];
+    const int a0 = (W.delta - gd.delta_min) + (gd.tmax - W.T);  // first tap of row 0 in the tile
+    W.q0 = a0 / D;
+    W.b0 = a0 - W.q0 * D;
+  }
+  // Long decimations: the windows of a row lie inside one period of D samples
+  // and leave gaps, which are not staged (64 taps of one phase at D = 320 read
+  // a fifth of the input) where that saves an eighth or more.
+  if (!gd.win && gd.delta_span + gd.tmax <= D) {
+    int lo[kMaxSegs], hi[kMaxSegs], ns = 0;
+    bool fits = true;
+    // union of the windows [b0, b0 + T): work sets in order of start, by
+    // repeated selection of the earliest start past the last segment
+    for (int at = 0; fits;) {
+      int best = INT32_MAX;
+      for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi)
+        if (L.ws[wi].b0 + L.ws[wi].T > at) best = std::min(best, std::max(at, L.ws[wi].b0));
+      if (best == INT32_MAX) break;
+      int end = best;
+      for (bool grew = true; grew;) {
+        grew = false;
+        for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi)
+          if (L.ws[wi].b0 <= end && L.ws[wi].b0 + L.ws[wi].T > end) {
+            end = L.ws[wi].b0 + L.ws[wi].T;
+            grew = true;
+          }
+      }
+      if (ns == kMaxSegs) {
+        fits = false;
+        break;
+      }
+      lo[ns] = best;
+      hi[ns++] = end;
+      at = end;
+    }
+    int nph = 0;
+    for (int i = 0; fits && i < ns; ++i) nph += hi[i] - lo[i];
+    if (fits && nph > 0 && 8 * nph <= 7 * D) {
+      for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) {
+        WorkSet<NB>& W = L.ws[wi];
+        int base = 0;
+        for (int i = 0; i < ns; base += hi[i] - lo[i], ++i)
+          if (W.b0 >= lo[i] && W.b0 < hi[i]) {
+            W.b0 = base + (W.b0 - lo[i]);
+            break;
+          }
+      }
+      // phase b of the row is staged sample b + seg_first + the gaps before it
+      gd.seg_first = lo[0];
+      for (int i = 1, at = hi[0] - lo[0]; i < ns; at += hi[i] - lo[i], ++i) {
+        gd.seg_at[i - 1] = at;
+        gd.seg_gap[i - 1] = lo[i] - hi[i - 1];
+      }
+      gd.nph = nph;
+      len = (int64_t)Qt * nph;
+    }
+  }
+  if (gd.nph == D) gd.seg_first = 0;
+  gd.len = (int32_t)len;
+  gd.step_q = kThreads / gd.nph;
+  gd.step_b = kThreads % gd.nph;
+  gd.span = (int32_t)(gd.nph == D ? len : (int64_t)Qt * D);
+  gd.inv_nph = ((1ull << 32) + (uint64_t)gd.nph - 1) / (uint64_t)gd.nph;  // exact quotients: len * nph < 2^32
+  int64_t P = (len + gd.nph - 1) / gd.nph;
+  if ((P & 1) == 0) P++;  // odd pitch: the staging scatter spreads over banks
+  gd.P = (int32_t)P;
+  // shared-memory layout: input tile | taps of each work set | channel constants
+  int64_t off = ((int64_t)gd.nph * P + 1) & ~1LL;  // float2 units, 16-byte aligned
+  gd.taps_off = (int32_t)off;
+  int64_t toff = 0;
+  for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) {
+    L.ws[wi].soff = (int32_t)toff;
+    toff += (int64_t)L.ws[wi].T * L.ws[wi].nb;
+  }
+  const int64_t meta_bytes = (int64_t)(gd.ws_end - gd.ws_begin) * NB * 48;
+  // taps go to shared memory unless they would push the CTA past ~150 KB
+  // (long filters of many phases); those groups read taps through L1
+  gd.taps_smem = ((off + 2 * toff) * (int64_t)sizeof(float2) + meta_bytes <= 150 * 1024) ? 1 : 0;
+  if (gd.taps_smem) off += 2 * toff;
+  gd.meta_off = (int32_t)off;
+  gd.smem_bytes = (int32_t)(off * (int64_t)sizeof(float2) + meta_bytes);
+}
+
 template <int NB>
 int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaStream_t stream) {
   static thread_local PolyLaunch<NB> L;  // ~20 KB: keep it off the stack
@@ -911,6 +1140,7 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
   L.block = in16_ ? nullptr : d_in;
   L.block16 = in16_;
   L.hist = d_hist_[hist_cur_];
+  L.new_hist = d_hist_[hist_cur_ ^ 1];
   L.N = (int64_t)n;
   L.H = H_;
   L.nco = d_nco_;
@@ -919,8 +1149,10 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
     const uint32_t R = chans_[c].nco.rollover;
     L.nco_base[c] = R ? (uint32_t)(abs0_ % R) : 0u;
   }
-  int ng = 0, nws = 0, max_tiles = 0;
-  size_t smem_max = 0;
+  int ng = 0, nws = 0;
+  int64_t rows_of[kMaxGroups];
+  int qt_of[kMaxGroups];
+  bool fixed_qt[kMaxGroups];
   for (auto& g : groups_) {
     GroupDesc& gd = L.groups[ng];
     gd.D = (int32_t)g.D;
@@ -939,7 +1171,7 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
         const uint32_t phi = (uint32_t)(t % U);
         if (nws >= kMaxWorkSets) return FDSP_ERR_UNSUPPORTED;
         WorkSet<NB>& W = L.ws[nws++];
-        W.taps = bt.d_taps + (size_t)phi * bt.T * ((bt.chans.size() + 1) & ~(size_t)1);
+        W.taps = bt.d_taps + (size_t)phi * bt.T * bt.chans.size();
         W.T = bt.T;
         W.delta = (int32_t)delta;
         W.J = (int32_t)J;
@@ -961,44 +1193,38 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
     // the sliding-window form where it fills the GPU with its larger tiles
     // (short blocks keep the per-row form, whose smaller tiles spread wider)
     const bool win = g.win && rows >= (int64_t)g.Qt_win * num_sms_;
-    const int Qt = win ? g.Qt_win : g.Qt;
-    gd.Qt = Qt;
     gd.win = win ? 1 : 0;
     gd.real_taps = g.real_taps;
-    gd.ntiles = (int32_t)((rows + Qt - 1) / Qt);
-    const int64_t len = (int64_t)Qt * g.D + gd.delta_span + tmax - 1;
-    int64_t P = (len + g.D - 1) / g.D;
-    if ((P & 1) == 0) P++;  // odd pitch: the staging scatter spreads over banks
-    gd.P = (int32_t)P;
-    // shared-memory layout: input tile | taps of each work set | channel constants
-    int64_t off = ((int64_t)g.D * P + 1) & ~1LL;  // float2 units, 16-byte aligned
-    gd.taps_off = (int32_t)off;
-    int64_t toff = 0;
-    for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) {
-      L.ws[wi].soff = (int32_t)toff;
-      toff += (int64_t)L.ws[wi].T * ((L.ws[wi].nb + 1) & ~1);
+    rows_of[ng] = rows;
+    qt_of[ng] = win ? g.Qt_win : g.Qt;
+    if (!win && g.Qt == g.Qt_default && g.Qt == 32) {  // two rows a thread where the windows' phases alone fit
+      layout_group<NB>(L, gd, 64);
+      if (gd.smem_bytes <= kSmem3) qt_of[ng] = 64;
     }
-    const int64_t meta_bytes = (int64_t)(gd.ws_end - gd.ws_begin) * NB * 48;
-    // taps go to shared memory unless they would push the CTA past ~150 KB
-    // (long filters of many phases); those groups read taps through L1
-    gd.taps_smem = ((off + toff) * (int64_t)sizeof(float2) + meta_bytes <= 150 * 1024) ? 1 : 0;
-    if (gd.taps_smem) off += toff;
-    gd.meta_off = (int32_t)off;
-    const int64_t bytes = off * (int64_t)sizeof(float2) + meta_bytes;
-    if (bytes > 227 * 1024) return FDSP_ERR_UNSUPPORTED;
-    gd.smem_bytes = (int32_t)bytes;
-    smem_max = std::max(smem_max, (size_t)bytes);
-    max_tiles = std::max(max_tiles, gd.ntiles);
+    fixed_qt[ng] = win || g.Qt != g.Qt_default;
     ng++;
   }
-  L.ngroups = ng;
-  L.max_tiles = max_tiles;
-  L.nws = nws;
-  if (num_sms_ == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, dev);
-    if (num_sms_ <= 0) num_sms_ = 1;
+  // Blocks too short to give every SM three tiles of the default height take
+  // lower tiles (latency: more of the GPU stages and computes at once).
+  for (int shift = 1; shift <= 5; ++shift) {
+    int64_t tiles = 0;
+    for (int gi = 0; gi < ng; ++gi) tiles += (rows_of[gi] + qt_of[gi] - 1) / qt_of[gi];
+    if (tiles >= 3LL * num_sms_) break;
+    for (int gi = 0; gi < ng; ++gi)
+      if (!fixed_qt[gi]) qt_of[gi] = std::max(32, (qt_of[gi] / 2) & ~31);
+  }
+  for (int gi = 0; gi < ng; ++gi) {
+    GroupDesc& gd = L.groups[gi];
+    for (;;) {  // a lower tile where this one leaves no room for two more CTAs (or is over the limit)
+      layout_group<NB>(L, gd, qt_of[gi]);
+      if (gd.smem_bytes <= (fixed_qt[gi] ? 227 * 1024 : kSmem3)) break;
+      if (gd.win || qt_of[gi] <= 32) {
+        if (gd.smem_bytes > 227 * 1024) return FDSP_ERR_UNSUPPORTED;
+        break;
+      }
+      qt_of[gi] -= 32;
+    }
+    gd.ntiles = (int32_t)((rows_of[gi] + gd.Qt - 1) / gd.Qt);
   }
   // tensor-core groups: one prep launch and one filter-bank launch for all of
   // them; groups the tensor-core plan cannot hold stay on the FP32 kernel
@@ -1018,76 +1244,86 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
       }
     }
   }
-  // small blocks: the FP32 groups in at most four launches (by way of
-  // staging taps and tile form; grid = tiles x groups, shared memory of the
-  // largest group of the launch); the per-launch cost then stops dominating
-  // short blocks
+  // The FP32 groups in one launch per kernel variant (taps staged or read
+  // through L1, sliding window or rows) and shared-memory size (three CTAs an
+  // SM or fewer), tallest work first; the last launch also writes the history.
+  // Group by group only for the autotuner, and for blocks of several waves
+  // whose outputs are copied back as groups finish (apply_host).
+  struct Batch {
+    const void* kern;
+    int first, count, tiles;
+    size_t smem;
+  };
+  Batch lb[kMaxGroups];
+  int nlb = 0, nm = 0;
   {
-    int nfp = 0;
-    int64_t tiles = 0;
+    int order[kMaxGroups], nfp = 0;
+    int64_t cost[kMaxGroups], tiles = 0;
     for (int gi = 0; gi < ng; ++gi) {
-      if (on_tc[gi] || L.groups[gi].ntiles <= 0) continue;
-      ++nfp;
-      tiles += L.groups[gi].ntiles;
+      const GroupDesc& gd = L.groups[gi];
+      if (on_tc[gi] || gd.ntiles <= 0) continue;
+      cost[gi] = 0;
+      for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) cost[gi] += (int64_t)L.ws[wi].T * L.ws[wi].nb * gd.Qt;
+      tiles += gd.ntiles;
+      order[nfp++] = gi;
     }
-    if (nfp > 1 && prof_ev_.empty() && tiles <= 3LL * num_sms_) {
-      int nm = 0;
-      for (int pass = 0; pass < 4; ++pass) {  // (taps in shared memory?, sliding window?)
-        const int first = nm;
-        size_t fsmem = 0;
-        int ftiles = 0;
-        const int want_smem = (pass & 1) == 0 ? 1 : 0, want_win = pass >> 1;
-        for (int gi = 0; gi < ng; ++gi) {
-          const GroupDesc& gd = L.groups[gi];
-          if (on_tc[gi] || gd.taps_smem != want_smem || gd.win != want_win || gd.ntiles <= 0) continue;
-          L.fuse_map[nm++] = (int8_t)gi;
-          fsmem = std::max(fsmem, (size_t)gd.smem_bytes);
-          ftiles = std::max(ftiles, (int)gd.ntiles);
+    std::sort(order, order + nfp, [&](int a, int b) { return cost[a] != cost[b] ? cost[a] > cost[b] : a < b; });
+    const bool single = !prof_ev_.empty() || (done_fn_ && tiles > 3LL * num_sms_);
+    for (int variant = 0; variant < 8; ++variant) {
+      const bool smem_taps = (variant & 1) == 0, win = (variant & 2) != 0, big = (variant & 4) != 0;
+      bool open = false;
+      for (int i = 0; i < nfp; ++i) {
+        const GroupDesc& gd = L.groups[order[i]];
+        if ((gd.taps_smem != 0) != smem_taps || (gd.win != 0) != win || (gd.smem_bytes > kSmem3) != big) continue;
+        if (!open || single) {
+          Batch& nb = lb[nlb++];
+          nb.kern = win ? (smem_taps ? reinterpret_cast<const void*>(poly_fp32_kernel<NB, true, true>)
+                                     : reinterpret_cast<const void*>(poly_fp32_kernel<NB, false, true>))
+                        : (smem_taps ? reinterpret_cast<const void*>(poly_fp32_kernel<NB, true, false>)
+                                     : reinterpret_cast<const void*>(poly_fp32_kernel<NB, false, false>));
+          nb.first = nm;
+          nb.count = nb.tiles = 0;
+          nb.smem = 0;
+          open = true;
         }
-        if (nm == first) continue;
-        auto kern = want_win ? (want_smem ? poly_fp32_kernel<NB, true, true> : poly_fp32_kernel<NB, false, true>)
-                             : (want_smem ? poly_fp32_kernel<NB, true, false> : poly_fp32_kernel<NB, false, false>);
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem);
-        if (e != cudaSuccess) return cuda_status(e);
-        if (kprof_) cudaEventRecord(kprof_event(), stream);
-        int garg = -1 - first;
-        e = klaunch(reinterpret_cast<const void*>(kern), dim3((unsigned)ftiles, (unsigned)(nm - first)),
-                    dim3(kThreads), fsmem, stream, L, garg);
-        if (kprof_) cudaEventRecord(kprof_event(), stream);
-        if (e != cudaSuccess) return cuda_status(e);
-        launches_last_++;
-        if (done_fn_) {
-          std::vector<int> egs;
-          for (int i = first; i < nm; ++i) egs.push_back(group_of_d_[L.groups[L.fuse_map[i]].D]);
-          notify_done(egs, stream);
-        }
+        Batch& cb = lb[nlb - 1];
+        L.fuse_map[nm++] = (int8_t)order[i];
+        cb.count++;
+        cb.tiles += gd.ntiles;
+        cb.smem = std::max(cb.smem, (size_t)gd.smem_bytes);
       }
-      for (int gi = 0; gi < ng; ++gi) on_tc[gi] = 1;  // nothing left for the per-group loop
     }
   }
-  // one launch per remaining FP32 group, each with its own tile shape and
-  // shared-memory size (all on `stream`, so they run back to back)
-  for (int gi = 0; gi < ng; ++gi) {
-    const GroupDesc& gd = L.groups[gi];
-    if (gd.ntiles <= 0 || on_tc[gi]) continue;
-    const int eg = group_of_d_[gd.D];
+  bool hist_done = false;
+  for (int li = 0; li < nlb; ++li) {
+    const Batch& bt = lb[li];
+    const int eg = group_of_d_[L.groups[L.fuse_map[bt.first]].D];
+    cudaError_t e = cudaFuncSetAttribute(bt.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt.smem);
+    if (e != cudaSuccess) return cuda_status(e);
     if (!prof_ev_.empty()) {
       cudaEventRecord(prof_ev_[2 * eg], stream);
       prof_hit_[eg] = 1;
     }
-    const size_t smem = (size_t)gd.smem_bytes;
-    auto kern = gd.win ? (gd.taps_smem ? poly_fp32_kernel<NB, true, true> : poly_fp32_kernel<NB, false, true>)
-                       : (gd.taps_smem ? poly_fp32_kernel<NB, true, false> : poly_fp32_kernel<NB, false, false>);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_status(e);
     if (kprof_) cudaEventRecord(kprof_event(), stream);
-    int garg = gi;
-    e = klaunch(reinterpret_cast<const void*>(kern), dim3((unsigned)gd.ntiles), dim3(kThreads), smem, stream, L, garg);
+    int first = bt.first, tiles = bt.tiles, hist_blocks = 0;
+    if (li + 1 == nlb && H_ > 0) {
+      hist_blocks = (H_ + kThreads - 1) / kThreads;
+      hist_done = true;
+    }
+    e = klaunch(bt.kern, dim3((unsigned)(tiles + hist_blocks)), dim3(kThreads), bt.smem, stream, L, first, tiles);
     if (kprof_) cudaEventRecord(kprof_event(), stream);
     if (e != cudaSuccess) return cuda_status(e);
     launches_last_++;
     if (!prof_ev_.empty()) cudaEventRecord(prof_ev_[2 * eg + 1], stream);
-    if (done_fn_) notify_done(std::vector<int>(1, eg), stream);
+    if (done_fn_) {
+      std::vector<int> egs;
+      for (int i = 0; i < bt.count; ++i) egs.push_back(group_of_d_[L.groups[L.fuse_map[bt.first + i]].D]);
+      notify_done(egs, stream);
+    }
+  }
+  if (hist_done) {
+    hist_cur_ ^= 1;
+    return FDSP_OK;
   }
   if (H_ > 0) {
     const float2* a0 = d_hist_[hist_cur_];

@@ -331,7 +331,7 @@ __device__ __noinline__ void tc_fix_exact(const TcLaunch& L, int slot, int64_t j
   cm.rollover = nc.rollover;
   cm.base = L.nco_base[S.ch];
   cm.enabled = nc.enabled;
-  cm.pad_ = 0;
+  cm.step32 = 0;
   const int64_t w0 = (int64_t)S.w0 + j * D;
   const ExactRot er = rotate_prep(cm, w0, S.T);
   float2 B = make_float2(0.f, 0.f);

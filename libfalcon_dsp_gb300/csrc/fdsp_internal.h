@@ -48,6 +48,8 @@ struct NcoConst {
 };
 
 // One decimation-factor group of an engine launch (one CTA per tile of it).
+constexpr int kMaxSegs = 4;  // runs of staged phases a row may have
+
 struct GroupDesc {
   int32_t D;          // down rate shared by every channel of the group
   int32_t Qt;         // output rows per tile (multiple of 32)
@@ -64,6 +66,15 @@ struct GroupDesc {
   int32_t taps_smem;  // 1: taps staged in shared memory; 0: read through L1
   int32_t win;        // 1: single-channel work sets, sliding-window rows (Qt multiple of 32 x kWinRows)
   int32_t real_taps;  // 1: every tap of the group is real (2 FMAs per tap)
+  int32_t rows;       // rows a thread computes in the row form (1, 2 or 4; Qt is a multiple of 32 rows)
+  int32_t len;        // staged samples of a tile
+  int32_t nph;        // staged phases of a row: D, or fewer where the windows leave gaps
+  int32_t seg_first;  // first staged phase of a row
+  int32_t seg_at[kMaxSegs - 1];   // staged phase where a gap lies (INT32_MAX: none)
+  int32_t seg_gap[kMaxSegs - 1];  // unstaged phases of that gap
+  int32_t step_q, step_b;  // kThreads staged samples on: rows and phases
+  int32_t span;       // input samples from the first staged one to past the last
+  uint64_t inv_nph;   // ceil(2^32 / nph): t / nph as one multiply and shift
 };
 
 // One (tap batch, output class r) pair of a launch.  Output j of the class is
@@ -71,14 +82,16 @@ struct GroupDesc {
 // [delta + j*D - T + 1, delta + j*D] in block-relative input indices.
 template <int NB>
 struct WorkSet {
-  const float2* taps;   // [T][nb] modulated taps of phase phi_r (device)
+  const float4* taps;   // [T][nb] modulated taps of phase phi_r, (re, re, im, im) (device)
   int32_t T;            // padded taps per phase of the batch
-  int32_t soff;         // shared-memory offset (float2) of these taps in the CTA
+  int32_t soff;         // offset (float4) of these taps in the CTA's staged taps
   int32_t delta;        // window end of row j = 0 (block relative)
   int32_t J;            // rows that have an output in this launch
   int32_t U;            // up rate of the batch's channels
   int32_t r;            // output class (m mod U)
   int32_t nb;           // live channels in the batch (<= NB)
+  int32_t b0;           // first tap of row 0 in the tile: staged phase
+  int32_t q0;           // and tile row
   int16_t ch[NB];       // channel ids
 };
 
@@ -87,13 +100,12 @@ struct PolyLaunch {
   const float2* block;      // device input block (N samples)
   const short2* block16;    // or, when set, the block as complex int16 (converted on load)
   const float2* hist;       // device history (H samples preceding block)
+  float2* new_hist;         // history of the next block (the last launch of an apply writes it)
   int64_t N;
   int32_t H;
-  int32_t ngroups;
-  int32_t max_tiles;
-  int32_t nws;
+  int32_t pad_;
   const NcoConst* nco;      // [nch]
-  int8_t fuse_map[kMaxGroups];  // fused launches: group of blockIdx.y + offset
+  int8_t fuse_map[kMaxGroups];  // groups in launch order: a launch takes the tiles of fuse_map[first ...]
   GroupDesc groups[kMaxGroups];
   WorkSet<NB> ws[kMaxWorkSets];
   float2* out[kMaxChannels];         // output base of each channel for this launch
@@ -223,7 +235,7 @@ struct EngineBatch {
   int group;           // decimation group index
   int T;               // padded taps per phase
   std::vector<int> chans;
-  float2* d_taps;      // [up][T][nb] on the device
+  float4* d_taps;      // [up][T][nb] on the device, (re, re, im, im)
 };
 
 struct EngineGroup {

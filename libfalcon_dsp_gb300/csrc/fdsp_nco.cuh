@@ -23,7 +23,7 @@ struct OutMeta {
   uint32_t rollover;  // R
   uint32_t base;      // counter of block sample 0 (mod R)
   uint32_t enabled;   // 0: no shift (phasor 1)
-  uint32_t pad_;
+  uint32_t step32;    // 32 D mod R: counter step of a thread's next row (FP32 engine)
 };
 
 __device__ __forceinline__ float2 cmul_nco(float2 a, float2 b) {
