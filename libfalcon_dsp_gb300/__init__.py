@@ -47,14 +47,31 @@ def _is_tensor(x) -> bool:
     return type(x).__module__.startswith("torch") and hasattr(x, "is_cuda")
 
 
+_torch_mod = None
+_raw_stream = None  # (device index) -> handle of its current stream
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_mod, _raw_stream
+    if _torch_mod is None:
+        import torch
+        _torch_mod = torch
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return _torch_mod
 
 
 def _stream_handle() -> int:
+    """Handle of the current stream of the current device (without building a
+    torch.cuda.Stream object: 0.3 us instead of 3)."""
     torch = _torch()
-    return torch.cuda.current_stream().cuda_stream
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
+
+
+def _head(t, n: int):
+    """The first n elements of t: t itself when that is all of it."""
+    return t if t.shape[0] == n else t[:n]
 
 
 def _c64(x) -> np.ndarray:
@@ -89,10 +106,10 @@ def _tptr(t) -> C.c_void_p:
 
 
 def _dev_c64(t):
-    torch = _torch()
-    if t.dtype != torch.complex64:
+    if t.dtype != _torch().complex64:
         raise TypeError("device input must be a complex64 CUDA tensor")
-    return t.contiguous().reshape(-1)
+    t = t.contiguous()
+    return t if t.dim() == 1 else t.reshape(-1)
 
 
 def freq_shift_params(fs: int, f: int) -> tuple[int, float]:
@@ -311,43 +328,43 @@ class MultiRateChannelizerCuda(_Handle):
         return [o[: n_out[i]] for i, o in enumerate(outs)]
 
     def _apply_ci16_device(self, x16, out, stream):
-        torch = _torch()
-        n = x16.shape[0]
-        if out is None:
-            out = [torch.empty(max(c, 1), dtype=torch.complex64, device=x16.device) for c in self.out_count(n)]
-        optr = (C.c_void_p * self.num_channels)(*[o.data_ptr() for o in out])
-        cap = (C.c_uint64 * self.num_channels)(*[o.numel() for o in out])
-        n_out = (C.c_uint64 * self.num_channels)()
-        s = _stream_handle() if stream is None else stream
-        _capi.call("fdsp_channelizer_apply_ci16", self._h, _tptr(x16), n, optr, cap, n_out, C.c_void_p(s))
-        return [o[: n_out[i]] for i, o in enumerate(out)]
+        return self._enqueue("fdsp_channelizer_apply_ci16", x16, x16.shape[0], out, stream)
 
     def _apply_device(self, x, out, stream):
-        torch = _torch()
         x = _dev_c64(x)
+        return self._enqueue("fdsp_channelizer_apply", x, x.numel(), out, stream)
+
+    def _enqueue(self, fn: str, x, n: int, out, stream):
+        torch = _torch()
         if out is None:
-            cnt = self.out_count(x.numel())
-            out = [torch.empty(max(c, 1), dtype=torch.complex64, device=x.device) for c in cnt]
-        # the ctypes pointer / capacity arrays are rebuilt only when the
-        # caller's output buffers change (streaming loops reuse them)
-        ptrs = tuple(o.data_ptr() for o in out)
+            out = [torch.empty(max(c, 1), dtype=torch.complex64, device=x.device) for c in self.out_count(n)]
+        # the ctypes arrays and the views of the output buffers are rebuilt
+        # when the caller's buffers change (streaming loops reuse them); a
+        # channel's count takes two values, so each channel keeps its views by
+        # count (slicing 64 outputs anew took 80 us a call)
+        ptrs = tuple(map(torch.Tensor.data_ptr, out))
+        sizes = tuple(map(torch.Tensor.numel, out))
         oc = getattr(self, "_out_cache", None)
-        if oc is None or oc[0] != ptrs:
-            n = self.num_channels
-            oc = (ptrs, (C.c_void_p * n)(*ptrs), (C.c_uint64 * n)(*[o.numel() for o in out]), (C.c_uint64 * n)())
+        if oc is None or oc[0] != ptrs or oc[1] != sizes:
+            k = self.num_channels
+            oc = (ptrs, sizes, (C.c_void_p * k)(*ptrs), (C.c_uint64 * k)(*sizes), (C.c_uint64 * k)(),
+                  [{} for _ in range(k)])
             self._out_cache = oc
-        _, optr, cap, n_out = oc
-        s = _stream_handle() if stream is None else stream
-        st = _capi.lib().fdsp_channelizer_apply(self._h, x.data_ptr(), x.numel(), optr, cap, n_out, s)
+        optr, cap, n_out, views = oc[2:]
+        st = getattr(_capi.lib(), fn)(self._h, x.data_ptr(), n, optr, cap, n_out,
+                                      _stream_handle() if stream is None else stream)
         if st:
-            _capi.check("fdsp_channelizer_apply", st)
-        # views of the output buffers, reused while the counts repeat
-        counts = tuple(n_out)
-        vc = getattr(self, "_view_cache", None)
-        if vc is None or vc[0] != ptrs or vc[1] != counts:
-            vc = (ptrs, counts, [o[:k] for o, k in zip(out, counts)])
-            self._view_cache = vc
-        return list(vc[2])
+            _capi.check(fn, st)
+        counts = n_out[:]
+        try:
+            return [v[c] for v, c in zip(views, counts)]
+        except KeyError:
+            for v, o, c in zip(views, out, counts):
+                if c not in v:
+                    if len(v) >= 4:
+                        v.clear()
+                    v[c] = o[:c]
+            return [v[c] for v, c in zip(views, counts)]
 
 
 class PolyphaseResamplerCuda(_Handle):
@@ -409,18 +426,22 @@ class PolyphaseResamplerCuda(_Handle):
 
     def apply(self, x, out=None, stream: int | None = None):
         if _is_tensor(x):
-            torch = _torch()
+            torch, lib = _torch(), _capi.lib()
             x16 = _ci16_dev(x)
             fn = "fdsp_resampler_apply_ci16" if x16 is not None else "fdsp_resampler_apply"
             x = x16 if x16 is not None else _dev_c64(x)
             n_in = x.shape[0] if x16 is not None else x.numel()
-            n = self.out_count(n_in)
-            if out is None:
-                out = torch.empty(max(n, 1), dtype=torch.complex64, device=x.device)
             got = C.c_uint64()
-            s = _stream_handle() if stream is None else stream
-            _capi.call(fn, self._h, _tptr(x), n_in, _tptr(out), out.numel(), C.byref(got), C.c_void_p(s))
-            return out[: got.value]
+            if out is None:
+                st = lib.fdsp_resampler_out_count(self._h, n_in, C.byref(got))
+                if st:
+                    _capi.check("fdsp_resampler_out_count", st)
+                out = torch.empty(max(got.value, 1), dtype=torch.complex64, device=x.device)
+            st = getattr(lib, fn)(self._h, x.data_ptr(), n_in, out.data_ptr(), out.numel(), C.byref(got),
+                                  _stream_handle() if stream is None else stream)
+            if st:
+                _capi.check(fn, st)
+            return _head(out, got.value)
         real_in = np.isrealobj(x) and np.asarray(x).dtype != np.int16
         xa = _c64(x)
         n = self.out_count(xa.size)
@@ -473,9 +494,11 @@ class FreqShiftCuda(_Handle):
                 out = [torch.empty((max(n, 1), 2), dtype=torch.int16, device=x16.device)
                        for _ in range(self.num_channels)]
             optr = (C.c_void_p * self.num_channels)(*[o.data_ptr() for o in out])
-            s = _stream_handle() if stream is None else stream
-            _capi.call("fdsp_freq_shift_apply_ci16", self._h, _tptr(x16), n, optr, C.c_void_p(s))
-            res = [o[:n] for o in out]
+            st = _capi.lib().fdsp_freq_shift_apply_ci16(self._h, x16.data_ptr(), n, optr,
+                                                        _stream_handle() if stream is None else stream)
+            if st:
+                _capi.check("fdsp_freq_shift_apply_ci16", st)
+            res = [_head(o, n) for o in out]
             return res[0] if self.single else res
         if not _is_tensor(x) and _ci16_host(x) is not None:
             x16 = _ci16_host(x)
@@ -488,13 +511,16 @@ class FreqShiftCuda(_Handle):
         if _is_tensor(x):
             torch = _torch()
             x = _dev_c64(x)
+            n = x.numel()
             if out is None:
-                out = [torch.empty(max(x.numel(), 1), dtype=torch.complex64, device=x.device)
+                out = [torch.empty(max(n, 1), dtype=torch.complex64, device=x.device)
                        for _ in range(self.num_channels)]
             optr = (C.c_void_p * self.num_channels)(*[o.data_ptr() for o in out])
-            s = _stream_handle() if stream is None else stream
-            _capi.call("fdsp_freq_shift_apply", self._h, _tptr(x), x.numel(), optr, C.c_void_p(s))
-            res = [o[: x.numel()] for o in out]
+            st = _capi.lib().fdsp_freq_shift_apply(self._h, x.data_ptr(), n, optr,
+                                                   _stream_handle() if stream is None else stream)
+            if st:
+                _capi.check("fdsp_freq_shift_apply", st)
+            res = [_head(o, n) for o in out]
         else:
             xa = _c64(x)
             res = [np.empty(max(xa.size, 1), np.complex64) for _ in range(self.num_channels)]
@@ -544,13 +570,18 @@ class FirFilterCuda(_Handle):
                 n = x16.shape[0]
                 if out is None:
                     out = torch.empty((max(n, 1), 2), dtype=torch.int16, device=x16.device)
-                _capi.call("fdsp_fir_apply_ci16", self._h, _tptr(x16), n, _tptr(out), C.c_void_p(s))
-                return out[:n]
+                st = _capi.lib().fdsp_fir_apply_ci16(self._h, x16.data_ptr(), n, out.data_ptr(), s)
+                if st:
+                    _capi.check("fdsp_fir_apply_ci16", st)
+                return _head(out, n)
             x = _dev_c64(x)
+            n = x.numel()
             if out is None:
-                out = torch.empty(max(x.numel(), 1), dtype=torch.complex64, device=x.device)
-            _capi.call("fdsp_fir_apply", self._h, _tptr(x), x.numel(), _tptr(out), C.c_void_p(s))
-            return out[: x.numel()]
+                out = torch.empty(max(n, 1), dtype=torch.complex64, device=x.device)
+            st = _capi.lib().fdsp_fir_apply(self._h, x.data_ptr(), n, out.data_ptr(), s)
+            if st:
+                _capi.check("fdsp_fir_apply", st)
+            return _head(out, n)
         x16 = _ci16_host(x)
         if x16 is not None:
             n = x16.shape[0]
@@ -582,9 +613,11 @@ class PolarDiscriminatorCuda(_Handle):
             if out is None:
                 out = torch.empty(max(x.numel(), 1), dtype=torch.float32, device=x.device)
             got = C.c_uint64()
-            s = _stream_handle() if stream is None else stream
-            _capi.call("fdsp_polar_apply", self._h, _tptr(x), x.numel(), _tptr(out), C.byref(got), C.c_void_p(s))
-            return out[: got.value]
+            st = _capi.lib().fdsp_polar_apply(self._h, x.data_ptr(), x.numel(), out.data_ptr(), C.byref(got),
+                                              _stream_handle() if stream is None else stream)
+            if st:
+                _capi.check("fdsp_polar_apply", st)
+            return _head(out, got.value)
         xa = _c64(x)
         y = np.empty(max(xa.size, 1), np.float32)
         got = C.c_uint64()
@@ -644,10 +677,11 @@ class FmDemodulatorCuda(_Handle):
             x = _dev_c64(x)
             if out is None:
                 out = torch.empty(max(n, 1), dtype=torch.int16, device=x.device)
-            s = _stream_handle() if stream is None else stream
-            _capi.call("fdsp_fm_demod_apply", self._h, _tptr(x), x.numel(), _tptr(out), out.numel(), C.byref(got),
-                       C.c_void_p(s))
-            return out[: got.value]
+            st = _capi.lib().fdsp_fm_demod_apply(self._h, x.data_ptr(), x.numel(), out.data_ptr(), out.numel(),
+                                                 C.byref(got), _stream_handle() if stream is None else stream)
+            if st:
+                _capi.check("fdsp_fm_demod_apply", st)
+            return _head(out, got.value)
         xa = _c64(x)
         y = np.empty(max(n, 1), np.int16)
         _capi.call("fdsp_fm_demod_apply_host", self._h, _ptr(xa), xa.size, _ptr(y), y.size, C.byref(got),
