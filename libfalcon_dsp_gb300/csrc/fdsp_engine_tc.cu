@@ -956,41 +956,34 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
     cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, dev);
     if (num_sms_ <= 0) num_sms_ = 1;
   }
-  // pack groups into launches
+  // Plan each group once, then fill launches with them in turn.  The row split
+  // is chosen when the block size, the slots or the split limit change (the
+  // choice plans every split: most of the planning time); between blocks of a
+  // stream only the windows' offsets move.
   std::vector<std::vector<int>> packs;  // indices into gin
   std::vector<TcPlan> plans;
-  {
-    std::vector<int> cur;
-    TcPlan cur_plan;
-    auto plan_of = [&](const std::vector<int>& idx, TcPlan& p) {
-      std::vector<TcGroupIn> sub;
-      for (int i : idx) sub.push_back(gin[i]);
-      return tc_plan(sub, (int64_t)n, H_, num_sms_, p) == 0;
-    };
-    for (int i = 0; i < (int)gin.size(); ++i) {
-      std::vector<int> trial = cur;
-      trial.push_back(i);
-      TcPlan p;
-      if (plan_of(trial, p)) {
-        cur = trial;
-        cur_plan = std::move(p);
-        continue;
+  for (int i = 0; i < (int)gin.size(); ++i) {
+    EngineGroup& eg = groups_[gmap[i]];
+    const bool known = eg.tc_plan_n == n && eg.tc_plan_slots == gin[i].slots.size() && eg.tc_plan_max == gin[i].max_split;
+    TcGroupPlan gp;
+    bool ok = known && tc_plan_group(gin[i], H_, eg.tc_plan_split, gp) == 0;
+    if (!ok) ok = tc_plan_group(gin[i], H_, 0, gp) == 0;
+    if (ok && !gp.ms.empty()) {
+      eg.tc_plan_n = n;
+      eg.tc_plan_slots = gin[i].slots.size();
+      eg.tc_plan_max = gin[i].max_split;
+      eg.tc_plan_split = gp.g.S;
+      if (plans.empty() || !tc_append(plans.back(), gp)) {
+        plans.emplace_back();
+        packs.emplace_back();
+        ok = tc_append(plans.back(), gp);
       }
-      if (!cur.empty()) {
-        packs.push_back(cur);
-        plans.push_back(std::move(cur_plan));
-      }
-      cur.assign(1, i);
-      if (!plan_of(cur, cur_plan)) {
-        fallback.push_back(gmap[i]);
-        cur.clear();
-      }
+      if (ok) packs.back().push_back(i);
     }
-    if (!cur.empty()) {
-      packs.push_back(cur);
-      plans.push_back(std::move(cur_plan));
-    }
+    if (!ok) fallback.push_back(gmap[i]);
   }
+  for (TcPlan& p : plans)
+    if (tc_finish(p, (int64_t)n, H_, num_sms_) != 0) return FDSP_ERR_UNSUPPORTED;
   if (plans.empty()) return FDSP_OK;
   if (plans.size() > (size_t)kTcMaxGroups) return FDSP_ERR_UNSUPPORTED;
   // scratch (grow only): the split input, which every pack reads, and the B

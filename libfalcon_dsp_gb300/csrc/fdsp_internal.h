@@ -245,6 +245,9 @@ struct EngineGroup {
   int use_tc = 1;      // tensor-core form when the precision asks for it (autotuned)
   int tc_split = 32;   // largest row split of the tensor-core form (1 = none)
   int tc_split_used = 1;  // row split of its last tensor-core launch
+  uint64_t tc_plan_n = 0;     // block size, slots and limit that tc_plan_split was chosen for
+  size_t tc_plan_slots = 0;
+  int tc_plan_max = 0, tc_plan_split = 0;
   int win = 0;         // single-channel long filters: the FP32 kernel's sliding-window form applies
   int Qt_win = 0;      // its tile rows (multiple of 32 x kWinRows)
   int real_taps = 0;   // every channel of the group has real taps

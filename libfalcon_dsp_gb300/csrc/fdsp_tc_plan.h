@@ -132,50 +132,62 @@ struct TcSlotX {
 // set and the next one of the same bundle).  Its width is its slot count:
 // bundles sit back to back, a one-slot bundle takes one column pair.
 struct TcBundle {
-  std::vector<TcSlotX> slots;
-  int64_t start;  // earliest window start of its slots
-  int64_t end;    // latest window end
+  int first, last;  // the channel's slots [first, last) of the sorted group (in output order, before the split)
+  int64_t start;    // earliest window start of its slots
+  int64_t end;      // latest window end
   int width;
 };
 
-inline std::vector<TcBundle> tc_bundles(const TcGroupIn& g, int S) {
-  std::vector<TcSlotX> xs;
-  for (const TcSlotIn& s : g.slots) {
-    for (int b = 0; b < S; ++b) {
+// The group's slots by channel and output offset: a bundle's slots are then
+// one range, whatever the split.
+inline std::vector<TcSlotIn> tc_sorted(const TcGroupIn& g) {
+  std::vector<TcSlotIn> xs = g.slots;
+  std::stable_sort(xs.begin(), xs.end(),
+                   [](const TcSlotIn& a, const TcSlotIn& b) { return a.ch != b.ch ? a.ch < b.ch : a.r < b.r; });
+  return xs;
+}
+
+// Calls fn(slot) for the slots of xs[first, last) under row split S, in output
+// order: rows j = S i + b become slot b, whose rows are S D apart.
+template <class Fn>
+inline void tc_split_slots(const std::vector<TcSlotIn>& xs, int first, int last, int D, int S, Fn&& fn) {
+  for (int b = 0; b < S; ++b)
+    for (int i = first; i < last; ++i) {
+      const TcSlotIn& s = xs[i];
       if (s.J <= b) continue;
       TcSlotX x;
       x.s = s;
-      x.s.delta = s.delta + (int64_t)b * g.D;
+      x.s.delta = s.delta + (int64_t)b * D;
       x.s.J = (s.J - b + S - 1) / S;
       x.s.U = s.U * S;
       x.s.r = s.r + b * s.U;
       x.start = x.s.delta - s.T + 1;
-      xs.push_back(x);
+      fn(x);
     }
-  }
-  std::stable_sort(xs.begin(), xs.end(), [](const TcSlotX& a, const TcSlotX& b) {
-    return a.s.ch != b.s.ch ? a.s.ch < b.s.ch : a.s.r < b.s.r;
-  });
-  std::vector<TcBundle> bs;
-  for (size_t i = 0; i < xs.size();) {
-    size_t j = i;
+}
+
+// Bundles of the sorted slots under row split S, by window start.
+inline void tc_bundles(const std::vector<TcSlotIn>& xs, int D, int S, std::vector<TcBundle>& bs) {
+  bs.clear();
+  for (int i = 0; i < (int)xs.size();) {
     TcBundle b;
-    b.start = xs[i].start;
-    b.end = xs[i].s.delta;
-    while (j < xs.size() && xs[j].s.ch == xs[i].s.ch) {
-      b.start = std::min(b.start, xs[j].start);
-      b.end = std::max(b.end, xs[j].s.delta);
-      b.slots.push_back(xs[j]);
-      ++j;
+    b.first = i;
+    b.start = INT64_MAX;
+    b.end = INT64_MIN;
+    b.width = 0;
+    for (; i < (int)xs.size() && xs[i].ch == xs[b.first].ch; ++i) {
+      const int n = (int)std::min<int64_t>(S, xs[i].J);  // slots of this output class
+      if (n <= 0) continue;
+      b.start = std::min(b.start, xs[i].delta - xs[i].T + 1);
+      b.end = std::max(b.end, xs[i].delta + (int64_t)(n - 1) * D);
+      b.width += n;
     }
-    b.width = (int)b.slots.size();
-    bs.push_back(b);
-    i = j;
+    b.last = i;
+    if (b.width > 0) bs.push_back(b);
   }
   std::stable_sort(bs.begin(), bs.end(), [](const TcBundle& a, const TcBundle& b) {
     return a.start != b.start ? a.start < b.start : a.end < b.end;
   });
-  return bs;
 }
 
 // Merge-set window of bundles [i, j) (sorted by start): its start in
@@ -229,22 +241,23 @@ inline int64_t tc_partition(const std::vector<TcBundle>& bs, int H, std::vector<
 // tiles (chunks per tile row x rows / S); ties keep the smaller split.  A
 // channel's bundle (U S slots) fits one merge set, and the group's slots
 // stay within four full merge sets.
-inline int tc_choose_split(const TcGroupIn& g, int H) {
+inline int tc_choose_split(const std::vector<TcSlotIn>& xs, int D, int max_split, int H) {
   int64_t J = 0;
   int Umax = 1;
-  for (const TcSlotIn& s : g.slots) {
+  for (const TcSlotIn& s : xs) {
     J = std::max(J, s.J);
     Umax = std::max(Umax, s.U);
   }
   int bestS = 0;
   double bestc = 0;
-  for (int S = 1; S <= std::max((g.D & 1) ? 2 : 1, g.max_split); S *= 2) {
-    if ((g.D & 1) && (S & 1)) continue;
+  std::vector<TcBundle> bs;
+  std::vector<size_t> cuts;
+  for (int S = 1; S <= std::max((D & 1) ? 2 : 1, max_split); S *= 2) {
+    if ((D & 1) && (S & 1)) continue;
     if ((int64_t)Umax * S > kTcMsetSlots) break;
-    if (S > 2 && (int64_t)g.slots.size() * S > 4 * kTcMsetSlots) break;
-    const std::vector<TcBundle> bs = tc_bundles(g, S);
+    if (S > 2 && (int64_t)xs.size() * S > 4 * kTcMsetSlots) break;
+    tc_bundles(xs, D, S, bs);
     if (bs.empty()) continue;
-    std::vector<size_t> cuts;
     const int64_t ch = tc_partition(bs, H, cuts);
     if (ch < 0) continue;
     const double c = (double)ch * (double)((J + (int64_t)S * kTcRows - 1) / ((int64_t)S * kTcRows));
@@ -256,83 +269,108 @@ inline int tc_choose_split(const TcGroupIn& g, int H) {
   return bestS;
 }
 
-// Returns 0 on success, -1 when the apply exceeds a launch's record limits
-// (the caller keeps those groups on the FP32 kernel).
-inline int tc_plan(const std::vector<TcGroupIn>& gin, int64_t N, int H, int num_sms, TcPlan& p) {
-  p = TcPlan();
-  int64_t wx_max = 0;
-  for (const TcGroupIn& g : gin) {
-    if (g.slots.empty()) continue;
-    const int S = tc_choose_split(g, H);
-    if (S == 0) return -1;
-    const int64_t Dp = (int64_t)S * g.D;
-    const std::vector<TcBundle> bs = tc_bundles(g, S);
-    if (bs.empty()) continue;
-    if ((int)p.groups.size() >= kTcMaxGroups) return -1;
-    const int gi = (int)p.groups.size();
-    TcPlanGroup pg;
-    pg.D = (int)Dp;
-    pg.S = S;
-    pg.Wx = 0;
-    std::vector<size_t> cuts;
-    if (tc_partition(bs, H, cuts) < 0) return -1;
-    for (size_t ci = 0; ci + 1 < cuts.size(); ++ci) {
-      const size_t i = cuts[ci], j = cuts[ci + 1];
-      int64_t a, nchunks;
-      tc_window(bs, i, j, H, &a, &nchunks);
-      int width = 0;
-      for (size_t q = i; q < j; ++q) width += bs[q].width;
-      // record field ranges (16-bit taps, strides and offsets)
-      if (nchunks * kTcChunkTaps > 65535) return -1;
-      for (size_t q = i; q < j; ++q)
-        for (const TcSlotX& x : bs[q].slots)
-          if (x.s.T > 65535 || x.s.U > 65535 || x.s.phi > 65535 || x.s.J > INT32_MAX) return -1;
-      const int NS = (int)tc_round_up(width, 8);
-      if ((int)p.ms.size() >= kTcMaxMsets || (int)p.slots.size() + NS > kTcMaxSlots) return -1;
-      TcMset m{};
-      m.a = (int32_t)a;
-      m.group = (int16_t)gi;
-      m.slot0 = (int16_t)p.slots.size();
-      m.NS = (int16_t)NS;
-      m.nchunks = (int16_t)nchunks;
-      m.R = (int16_t)(4 * NS <= 128 ? 2 : 1);
-      int64_t Jmax = 0;
-      for (size_t q = i; q < j; ++q) {
-        const TcBundle& b = bs[q];
-        const size_t pos0 = p.slots.size() - (size_t)m.slot0;  // the bundle's first position in the merge set
-        for (size_t k = 0; k < b.slots.size(); ++k) {
-          const TcSlotX& x = b.slots[k];
-          TcSlot s{};
-          s.w0 = (int32_t)x.start;
-          s.J = (int32_t)x.s.J;
-          s.ch = (uint16_t)x.s.ch;
-          s.T = (uint16_t)x.s.T;
-          s.U = (uint16_t)x.s.U;
-          s.o = (uint16_t)(x.start + H - a);
-          s.phi = (uint16_t)x.s.phi;
-          // a slot at an even position followed by the channel's next output:
-          // one 16-byte store
-          s.flags = ((pos0 + k) % 2 == 0 && k + 1 < b.slots.size() && b.slots[k + 1].s.r == x.s.r + 1) ? 1 : 0;
-          p.slots.push_back(s);
-          p.slot_r.push_back(x.s.r);
-          Jmax = std::max(Jmax, x.s.J);
-        }
-      }
-      for (int q = width; q < NS; ++q) {
-        p.slots.push_back(TcSlot{});
-        p.slot_r.push_back(0);
-      }
-      m.ntiles = (int32_t)((Jmax + kTcRows - 1) / kTcRows);
-      m.items = (m.ntiles + m.R - 1) / m.R;
-      m.b = p.b_bytes;
-      p.b_bytes += (size_t)tc_round_up((int64_t)m.nchunks * 4 * NS * 128, 1024);
-      pg.Wx = std::max<int64_t>(pg.Wx, a % Dp + (int64_t)m.nchunks * kTcChunkTaps);
-      p.ms.push_back(m);
+// One group planned by itself: its merge sets (group 0, slots and B image
+// counted from 0), to be placed into a launch by tc_append.
+struct TcGroupPlan {
+  TcPlanGroup g;
+  std::vector<TcMset> ms;
+  std::vector<TcSlot> slots;
+  std::vector<int> slot_r;
+  size_t b_bytes = 0;
+};
+
+// Plans a group; S: its row split, or 0 to choose one.  Returns 0, or -1 when
+// the group exceeds a launch's record limits by itself.  A group without
+// outputs gives a plan without merge sets.
+inline int tc_plan_group(const TcGroupIn& g, int H, int S, TcGroupPlan& q) {
+  q = TcGroupPlan();
+  const std::vector<TcSlotIn> xs = tc_sorted(g);
+  if (S == 0) S = tc_choose_split(xs, g.D, g.max_split, H);
+  if (S == 0) return -1;
+  const int64_t Dp = (int64_t)S * g.D;
+  q.g.D = (int)Dp;
+  q.g.S = S;
+  q.g.Wx = 0;
+  std::vector<TcBundle> bs;
+  std::vector<size_t> cuts;
+  tc_bundles(xs, g.D, S, bs);
+  if (bs.empty()) return 0;
+  if (tc_partition(bs, H, cuts) < 0) return -1;
+  for (size_t ci = 0; ci + 1 < cuts.size(); ++ci) {
+    const size_t i = cuts[ci], j = cuts[ci + 1];
+    int64_t a, nchunks;
+    tc_window(bs, i, j, H, &a, &nchunks);
+    int width = 0;
+    for (size_t b = i; b < j; ++b) width += bs[b].width;
+    if (nchunks * kTcChunkTaps > 65535) return -1;  // record field ranges (16-bit taps, strides and offsets)
+    const int NS = (int)tc_round_up(width, 8);
+    if ((int)q.ms.size() >= kTcMaxMsets || (int)q.slots.size() + NS > kTcMaxSlots) return -1;
+    TcMset m{};
+    m.a = (int32_t)a;
+    m.slot0 = (int16_t)q.slots.size();
+    m.NS = (int16_t)NS;
+    m.nchunks = (int16_t)nchunks;
+    m.R = (int16_t)(4 * NS <= 128 ? 2 : 1);
+    int64_t Jmax = 0;
+    bool range = true;
+    for (size_t b = i; b < j; ++b) {
+      const size_t n0 = q.slots.size();  // the bundle's first slot
+      tc_split_slots(xs, bs[b].first, bs[b].last, g.D, S, [&](const TcSlotX& x) {
+        if (x.s.T > 65535 || x.s.U > 65535 || x.s.phi > 65535 || x.s.J > INT32_MAX) range = false;
+        TcSlot s{};
+        s.w0 = (int32_t)x.start;
+        s.J = (int32_t)x.s.J;
+        s.ch = (uint16_t)x.s.ch;
+        s.T = (uint16_t)x.s.T;
+        s.U = (uint16_t)x.s.U;
+        s.o = (uint16_t)(x.start + H - a);
+        s.phi = (uint16_t)x.s.phi;
+        q.slots.push_back(s);
+        q.slot_r.push_back(x.s.r);
+        Jmax = std::max(Jmax, x.s.J);
+      });
+      // a slot at an even position followed by the channel's next output: one
+      // 16-byte store
+      for (size_t k = n0; k + 1 < q.slots.size(); ++k)
+        q.slots[k].flags = ((k - (size_t)m.slot0) % 2 == 0 && q.slot_r[k + 1] == q.slot_r[k] + 1) ? 1 : 0;
     }
-    wx_max = std::max(wx_max, pg.Wx);
-    p.groups.push_back(pg);
+    if (!range) return -1;
+    q.slots.resize((size_t)m.slot0 + NS, TcSlot{});
+    q.slot_r.resize((size_t)m.slot0 + NS, 0);
+    m.ntiles = (int32_t)((Jmax + kTcRows - 1) / kTcRows);
+    m.items = (m.ntiles + m.R - 1) / m.R;
+    m.b = q.b_bytes;
+    q.b_bytes += (size_t)tc_round_up((int64_t)m.nchunks * 4 * NS * 128, 1024);
+    q.g.Wx = std::max<int64_t>(q.g.Wx, a % Dp + (int64_t)m.nchunks * kTcChunkTaps);
+    q.ms.push_back(m);
   }
+  return 0;
+}
+
+// Adds a planned group to launch p; false when the launch's records are full.
+inline bool tc_append(TcPlan& p, const TcGroupPlan& q) {
+  if (p.groups.size() >= (size_t)kTcMaxGroups || p.ms.size() + q.ms.size() > (size_t)kTcMaxMsets ||
+      p.slots.size() + q.slots.size() > (size_t)kTcMaxSlots)
+    return false;
+  for (TcMset m : q.ms) {
+    m.group = (int16_t)p.groups.size();
+    m.slot0 = (int16_t)(m.slot0 + p.slots.size());
+    m.b += p.b_bytes;
+    p.ms.push_back(m);
+  }
+  p.groups.push_back(q.g);
+  p.slots.insert(p.slots.end(), q.slots.begin(), q.slots.end());
+  p.slot_r.insert(p.slot_r.end(), q.slot_r.begin(), q.slot_r.end());
+  p.b_bytes += q.b_bytes;
+  return true;
+}
+
+// Sizes and schedule of a launch whose groups are all added.  Returns 0, or
+// -1 when its stages do not fit shared memory.
+inline int tc_finish(TcPlan& p, int64_t N, int H, int num_sms) {
   if (p.ms.empty()) return 0;
+  int64_t wx_max = 0;
+  for (const TcPlanGroup& g : p.groups) wx_max = std::max(wx_max, g.Wx);
   // the split writes [history | block] and a zero tail: every row a tensor
   // map can address ((rows - 1) D' + Wx samples) stays inside it
   p.xhl_samples = tc_round_up(N + H + wx_max + 16, 16);
@@ -357,6 +395,19 @@ inline int tc_plan(const std::vector<TcGroupIn>& gin, int64_t N, int H, int num_
   p.G = (int)std::max<int64_t>(1, std::min<int64_t>(num_sms, p.items));
   p.Lc = (umax + p.G - 1) / p.G;
   return 0;
+}
+
+// Every group in one launch.  Returns 0 on success, -1 when they exceed a
+// launch's record limits.
+inline int tc_plan(const std::vector<TcGroupIn>& gin, int64_t N, int H, int num_sms, TcPlan& p) {
+  p = TcPlan();
+  TcGroupPlan q;
+  for (const TcGroupIn& g : gin) {
+    if (g.slots.empty()) continue;
+    if (tc_plan_group(g, H, 0, q) != 0) return -1;
+    if (!q.ms.empty() && !tc_append(p, q)) return -1;
+  }
+  return tc_finish(p, N, H, num_sms);
 }
 
 // Item range [first, last) of merge set m owned by CTA b (shared with the
