@@ -30,6 +30,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <type_traits>
 
 #include "fdsp_internal.h"
 #include "fdsp_nco.cuh"
@@ -555,6 +556,114 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
   }
 }
 
+// Rational resampling of one unshifted channel with many output phases
+// (U >= kNatMinUp): consecutive outputs on consecutive lanes.  Their windows
+// start D / U samples apart, so sample reads of the tile as it lies in memory
+// hardly conflict, the taps lie in output order (column r of [T][U]: phase r D
+// mod U; conflict-free, staged as they lie), and stores are contiguous.  The row form gives each of the U phases its own work
+// set: outputs U apart on neighbouring lanes (a sector per 8-byte store) and a
+// tile 160 x 34 samples that leaves one CTA an SM.  Bound: shared-memory reads
+// (a sample and a tap per multiply-add pair).  147/160 of 2^20 samples, 24 taps
+// a phase: 31 us in row form, 12 us here.  Sums run in the row form's order.
+// kCheck keeps that form's products with the taps' zero imaginary parts: an
+// infinite or NaN sample then marks both parts of an output, as it did there.
+constexpr int kNatMinUp = 16;
+constexpr int kNatMaxTaps = 8192;  // U T: 32 KB of taps in shared memory
+constexpr int kNatPer = 4;         // outputs a thread of a full tile
+
+template <bool kCheck>
+__global__ void __launch_bounds__(kThreads) nat_resample_kernel(const __grid_constant__ NatLaunch L, int tiles) {
+  extern __shared__ __align__(16) float2 xs[];
+  if ((int)blockIdx.x >= tiles) {
+    const int i = ((int)blockIdx.x - tiles) * kThreads + (int)threadIdx.x;
+    if (i < L.H) hist_sample(L.hist, L.block, L.block16, L.N, L.H, L.new_hist, i);
+    return;
+  }
+  const int U = L.U, D = L.D, T = L.T, per = L.per;
+  const int64_t m0 = (int64_t)blockIdx.x * (per * kThreads);
+  const int count = (int)min((int64_t)per * kThreads, L.M - m0);
+  const uint64_t t0 = (uint64_t)L.phase + (uint64_t)m0 * (uint64_t)D;
+  const int64_t s0 = L.xoffset + (int64_t)(t0 / U) - T + 1;  // first sample of output m0's window
+  const uint32_t ph0 = (uint32_t)(t0 % U);
+  const int r0 = L.r_first + (int)(m0 % U);
+  float* const taps = reinterpret_cast<float*>(xs + L.len);
+  const int len = (int)((ph0 + (uint64_t)(count - 1) * D) / U) + T;  // samples the outputs read (<= L.len)
+  for (int i = threadIdx.x; i < len; i += kThreads) {
+    const int64_t v = s0 + i;
+    if (L.block16 == nullptr) {
+      const float2* src = L.block;
+      uint32_t bytes = 0;
+      if (v < 0) {
+        if (v + L.H >= 0) {
+          src = L.hist + (v + L.H);
+          bytes = 8;
+        }
+      } else if (v < L.N) {
+        src = L.block + v;
+        bytes = 8;
+      }
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(
+                       (uint32_t)__cvta_generic_to_shared(xs + i)),
+                   "l"(src), "r"(bytes)
+                   : "memory");
+    } else {
+      float2 x = make_float2(0.f, 0.f);
+      if (v < 0) {
+        if (v + L.H >= 0) x = L.hist[v + L.H];
+      } else if (v < L.N) {
+        const short2 s = L.block16[v];
+        x = make_float2((float)s.x, (float)s.y);
+      }
+      xs[i] = x;
+    }
+  }
+  for (int i = threadIdx.x; i < (U * T + 3) / 4; i += kThreads)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(taps) + 16u * (uint32_t)i),
+                 "l"(reinterpret_cast<const float4*>(L.taps) + i)
+                 : "memory");
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+
+  const f32x2* xp[kNatPer];
+  const float* tp[kNatPer];
+  f32x2 acc[kNatPer], chk[kNatPer];
+#pragma unroll
+  for (int q = 0; q < kNatPer; ++q) {
+    const int l = min((int)threadIdx.x + q * kThreads, count - 1);  // (past the end: a valid window, not stored)
+    xp[q] = reinterpret_cast<const f32x2*>(xs) + (ph0 + (uint32_t)l * (uint32_t)D) / (uint32_t)U;
+    tp[q] = taps + (uint32_t)(r0 + l) % (uint32_t)U;  // column of output m0 + l
+    acc[q] = chk[q] = 0ull;
+  }
+  auto sum = [&](auto outs) {
+    constexpr int kOuts = decltype(outs)::value;
+#pragma unroll 4
+    for (int k = 0; k < T; ++k) {
+#pragma unroll
+      for (int q = 0; q < kOuts; ++q) {
+        const f32x2 x = xp[q][k];
+        const float h = tp[q][k * U];
+        acc[q] = fma2(pack2(h, h), x, acc[q]);
+        if constexpr (kCheck) chk[q] = fma2(0ull, x, chk[q]);
+      }
+    }
+  };
+  if (per == kNatPer) sum(std::integral_constant<int, kNatPer>());
+  else sum(std::integral_constant<int, 1>());
+#pragma unroll
+  for (int q = 0; q < kNatPer; ++q) {
+    const int l = (int)threadIdx.x + q * kThreads;
+    if (q >= per || l >= count) continue;
+    float2 y = unpack2(acc[q]);
+    if constexpr (kCheck) {
+      const float2 z = unpack2(chk[q]);
+      y = make_float2(y.x - z.y, y.y + z.x);
+    }
+    L.out[m0 + l] = y;
+  }
+}
+
 // The history update alone (applies whose groups all ran on the tensor cores).
 __global__ void hist_update_kernel(const float2* __restrict__ old_hist, const float2* __restrict__ block,
                                    const short2* __restrict__ block16, int64_t N, int H, float2* __restrict__ new_hist) {
@@ -595,6 +704,7 @@ PolyEngine::~PolyEngine() {
     if (b.d_taps) dfree(b.d_taps);
   }
   if (d_nco_) dfree(d_nco_);
+  if (d_nat_) dfree(d_nat_);
   for (auto& h : d_hist_) {
     if (h) dfree(h);
   }
@@ -820,6 +930,31 @@ int PolyEngine::init(uint32_t fs, const fdsp_channel_cfg* ch, uint32_t nch, bool
     cudaError_t e = dalloc(reinterpret_cast<void**>(&bt.d_taps), host.size() * sizeof(float4));
     if (e != cudaSuccess) return cuda_status(e);
     e = cudaMemcpy(bt.d_taps, host.data(), host.size() * sizeof(float4), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return cuda_status(e);
+  }
+
+  // one unshifted channel of many phases, every phase in turn (up and down
+  // coprime), whose windows move slowly (a tile of outputs spans at most 4
+  // samples an output): the many-phase form, its taps in output order
+  const uint32_t U0 = chans_[0].up, D0 = chans_[0].down;
+  uint32_t g0 = U0;
+  for (uint32_t b = D0, r; b; b = r) {
+    r = g0 % b;
+    g0 = b;
+  }
+  if (nch == 1 && !complex_taps && !chans_[0].nco.enabled && U0 >= (uint32_t)kNatMinUp && g0 == 1 && D0 <= 4u * U0 &&
+      (uint64_t)U0 * chans_[0].T <= (uint64_t)kNatMaxTaps) {
+    const uint32_t T0 = chans_[0].T;
+    std::vector<float> host(((size_t)U0 * T0 + 3) & ~(size_t)3, 0.f);
+    nat_col_.assign(U0, 0);
+    for (uint32_t r = 0; r < U0; ++r) {
+      const uint32_t phi = (uint32_t)((uint64_t)r * D0 % U0);
+      nat_col_[phi] = (int32_t)r;
+      for (uint32_t k = 0; k < T0; ++k) host[(size_t)k * U0 + r] = chans_[0].flipped[(size_t)phi * T0 + k].x;
+    }
+    cudaError_t e = dalloc(reinterpret_cast<void**>(&d_nat_), host.size() * sizeof(float));
+    if (e != cudaSuccess) return cuda_status(e);
+    e = cudaMemcpy(d_nat_, host.data(), host.size() * sizeof(float), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_status(e);
   }
 
@@ -1244,6 +1379,8 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
       }
     }
   }
+  if (d_nat_ && ng == 1 && !on_tc[0] && prof_ev_.empty())
+    return launch_nat(d_in, n, out[0], L.groups[0].win == 0, stream);
   // The FP32 groups in one launch per kernel variant (taps staged or read
   // through L1, sliding window or rows) and shared-memory size (three CTAs an
   // SM or fewer), tallest work first; the last launch also writes the history.
@@ -1338,6 +1475,47 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
     hist_cur_ ^= 1;
     launches_last_++;
   }
+  return FDSP_OK;
+}
+
+// The many-phase form of the engine's only channel.
+int PolyEngine::launch_nat(const float2* d_in, uint64_t n, float2* out, bool check, cudaStream_t stream) {
+  const EngineClass& k = classes_[0];
+  NatLaunch L;
+  std::memset(&L, 0, sizeof(L));
+  L.block = in16_ ? nullptr : d_in;
+  L.block16 = in16_;
+  L.hist = d_hist_[hist_cur_];
+  L.new_hist = d_hist_[hist_cur_ ^ 1];
+  L.taps = d_nat_;
+  L.r_first = nat_col_[k.phase];
+  L.out = out;
+  L.N = (int64_t)n;
+  L.M = (int64_t)k.M;
+  L.xoffset = (int64_t)k.xoffset;
+  L.phase = k.phase;
+  L.U = (int32_t)k.up;
+  L.D = (int32_t)k.down;
+  L.T = batches_[0].T;
+  L.H = H_;
+  // full tiles where they give every SM two, one output a thread otherwise
+  L.per = L.M >= 2LL * num_sms_ * kNatPer * kThreads ? kNatPer : 1;
+  const int64_t outs = (int64_t)L.per * kThreads;
+  L.len = (int32_t)((((outs - 1) * L.D + L.U - 1) / L.U + L.T + 1) & ~1LL);
+  const size_t smem = (size_t)L.len * sizeof(float2) + (((size_t)L.U * L.T + 3) & ~(size_t)3) * sizeof(float);
+  int tiles = (int)((L.M + outs - 1) / outs);
+  const int hist_blocks = (H_ + kThreads - 1) / kThreads;
+  const void* kern = check ? reinterpret_cast<const void*>(nat_resample_kernel<true>)
+                           : reinterpret_cast<const void*>(nat_resample_kernel<false>);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return cuda_status(e);
+  if (kprof_) cudaEventRecord(kprof_event(), stream);
+  e = klaunch(kern, dim3((unsigned)(tiles + hist_blocks)), dim3(kThreads), smem, stream, L, tiles);
+  if (kprof_) cudaEventRecord(kprof_event(), stream);
+  if (e != cudaSuccess) return cuda_status(e);
+  launches_last_++;
+  if (H_ > 0) hist_cur_ ^= 1;
+  if (done_fn_) notify_done(std::vector<int>(1, 0), stream);
   return FDSP_OK;
 }
 

@@ -112,6 +112,23 @@ struct PolyLaunch {
   uint32_t nco_base[kMaxChannels];   // (samples since reset at block[0]) mod R
 };
 
+// One channel of many output phases (nat_resample_kernel).
+struct NatLaunch {
+  const float2* block;      // device input block (N samples)
+  const short2* block16;    // or, when set, the block as complex int16
+  const float2* hist;       // device history (H samples preceding block)
+  float2* new_hist;         // history of the next block
+  const float* taps;        // [T][U], column r the taps of phase r D mod U
+  float2* out;
+  int64_t N, M;             // input samples, outputs
+  int64_t xoffset;          // state at the block's start
+  uint32_t phase;
+  int32_t r_first;          // column of output 0
+  int32_t U, D, T, H;
+  int32_t per;              // outputs a thread
+  int32_t len;              // samples a tile stages at most
+};
+
 // ---------------------------------------------------------------------------
 // Tensor-core launch: the decimation groups of one launch pack computed on
 // the tensor cores, planned by tc_plan (fdsp_tc_plan.h).  The record is the
@@ -352,6 +369,9 @@ class PolyEngine {
  private:
   template <int NB>
   int launch(const float2* d_in, uint64_t n, float2* const* out, cudaStream_t stream);
+  int launch_nat(const float2* d_in, uint64_t n, float2* out, bool check, cudaStream_t stream);
+  float* d_nat_ = nullptr;             // many-phase form: its taps (nullptr: the engine is not of that kind)
+  std::vector<int32_t> nat_col_;       // column of a tap phase
   int build_tc(int fmt);
   void free_tc();
   int launch_tc(const float2* d_in, uint64_t n, float2* const* out, const std::vector<int>& tc_groups,
