@@ -563,32 +563,33 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
 // mod U; conflict-free, staged as they lie), and stores are contiguous.  The row form gives each of the U phases its own work
 // set: outputs U apart on neighbouring lanes (a sector per 8-byte store) and a
 // tile 160 x 34 samples that leaves one CTA an SM.  Bound: shared-memory reads
-// (a sample and a tap per multiply-add pair).  147/160 of 2^20 samples, 24 taps
-// a phase: 31 us in row form, 12 us here.  Sums run in the row form's order.
+// (a sample per output and tap; a tap read feeds the thread's four outputs,
+// whose windows lie whole periods apart).  147/160 of 2^20 samples, 24 taps
+// a phase: 31 us in row form, 17 us here (cold cache).  Sums run in the row form's order.
 // kCheck keeps that form's products with the taps' zero imaginary parts: an
 // infinite or NaN sample then marks both parts of an output, as it did there.
 constexpr int kNatMinUp = 16;
 constexpr int kNatMaxTaps = 8192;  // U T: 32 KB of taps in shared memory
 constexpr int kNatPer = 4;         // outputs a thread of a full tile
+constexpr int kNatMaxCols = 512;   // threads of a CTA: a multiple of U columns, rounded up to warps
 
 template <bool kCheck>
-__global__ void __launch_bounds__(kThreads) nat_resample_kernel(const __grid_constant__ NatLaunch L, int tiles) {
+__global__ void __launch_bounds__(kNatMaxCols) nat_resample_kernel(const __grid_constant__ NatLaunch L, int tiles) {
   extern __shared__ __align__(16) float2 xs[];
+  const int threads = (int)blockDim.x;
   if ((int)blockIdx.x >= tiles) {
-    const int i = ((int)blockIdx.x - tiles) * kThreads + (int)threadIdx.x;
+    const int i = ((int)blockIdx.x - tiles) * threads + (int)threadIdx.x;
     if (i < L.H) hist_sample(L.hist, L.block, L.block16, L.N, L.H, L.new_hist, i);
     return;
   }
-  const int U = L.U, D = L.D, T = L.T, per = L.per;
-  const int64_t m0 = (int64_t)blockIdx.x * (per * kThreads);
-  const int count = (int)min((int64_t)per * kThreads, L.M - m0);
-  const uint64_t t0 = (uint64_t)L.phase + (uint64_t)m0 * (uint64_t)D;
-  const int64_t s0 = L.xoffset + (int64_t)(t0 / U) - T + 1;  // first sample of output m0's window
-  const uint32_t ph0 = (uint32_t)(t0 % U);
-  const int r0 = L.r_first + (int)(m0 % U);
+  const int U = L.U, D = L.D, T = L.T, cols = L.cols;
+  const int64_t m0 = (int64_t)blockIdx.x * (L.per * cols);  // a multiple of U: every tile starts at the same phase
+  const int count = (int)min((int64_t)L.per * cols, L.M - m0);
+  const int64_t s0 = L.xoffset + (m0 / U) * D - T + 1;  // first sample of output m0's window
+  const uint32_t ph0 = L.phase;
   float* const taps = reinterpret_cast<float*>(xs + L.len);
   const int len = (int)((ph0 + (uint64_t)(count - 1) * D) / U) + T;  // samples the outputs read (<= L.len)
-  for (int i = threadIdx.x; i < len; i += kThreads) {
+  for (int i = threadIdx.x; i < len; i += threads) {
     const int64_t v = s0 + i;
     if (L.block16 == nullptr) {
       const float2* src = L.block;
@@ -617,7 +618,7 @@ __global__ void __launch_bounds__(kThreads) nat_resample_kernel(const __grid_con
       xs[i] = x;
     }
   }
-  for (int i = threadIdx.x; i < (U * T + 3) / 4; i += kThreads)
+  for (int i = threadIdx.x; i < (U * T + 3) / 4; i += threads)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(
                      (uint32_t)__cvta_generic_to_shared(taps) + 16u * (uint32_t)i),
                  "l"(reinterpret_cast<const float4*>(L.taps) + i)
@@ -626,42 +627,45 @@ __global__ void __launch_bounds__(kThreads) nat_resample_kernel(const __grid_con
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
 
-  const f32x2* xp[kNatPer];
-  const float* tp[kNatPer];
-  f32x2 acc[kNatPer], chk[kNatPer];
-#pragma unroll
-  for (int q = 0; q < kNatPer; ++q) {
-    const int l = min((int)threadIdx.x + q * kThreads, count - 1);  // (past the end: a valid window, not stored)
-    xp[q] = reinterpret_cast<const f32x2*>(xs) + (ph0 + (uint32_t)l * (uint32_t)D) / (uint32_t)U;
-    tp[q] = taps + (uint32_t)(r0 + l) % (uint32_t)U;  // column of output m0 + l
-    acc[q] = chk[q] = 0ull;
-  }
-  auto sum = [&](auto outs) {
+  // column c of the tile: outputs c, c + cols, ..., whose windows lie
+  // cols / U * D samples apart and share their taps
+  const int c = (int)threadIdx.x;
+  if (c >= cols || c >= count) return;
+  const f32x2* xp = reinterpret_cast<const f32x2*>(xs) + (ph0 + (uint32_t)c * (uint32_t)D) / (uint32_t)U;
+  const float* tp = taps + (uint32_t)(L.r_first + c) % (uint32_t)U;
+  auto run = [&](auto outs) {
     constexpr int kOuts = decltype(outs)::value;
-#pragma unroll 4
+    f32x2 acc[kOuts], chk[kOuts];
+    int off[kOuts];
+#pragma unroll
+    for (int q = 0; q < kOuts; ++q) {
+      off[q] = c + q * cols < count ? q * (cols / U * D) : 0;  // (past the end: a valid window, not stored)
+      acc[q] = chk[q] = 0ull;
+    }
+#pragma unroll 2
     for (int k = 0; k < T; ++k) {
+      const float h = tp[k * U];
+      const f32x2 hh = pack2(h, h);
 #pragma unroll
       for (int q = 0; q < kOuts; ++q) {
-        const f32x2 x = xp[q][k];
-        const float h = tp[q][k * U];
-        acc[q] = fma2(pack2(h, h), x, acc[q]);
+        const f32x2 x = xp[k + off[q]];
+        acc[q] = fma2(hh, x, acc[q]);
         if constexpr (kCheck) chk[q] = fma2(0ull, x, chk[q]);
       }
     }
-  };
-  if (per == kNatPer) sum(std::integral_constant<int, kNatPer>());
-  else sum(std::integral_constant<int, 1>());
 #pragma unroll
-  for (int q = 0; q < kNatPer; ++q) {
-    const int l = (int)threadIdx.x + q * kThreads;
-    if (q >= per || l >= count) continue;
-    float2 y = unpack2(acc[q]);
-    if constexpr (kCheck) {
-      const float2 z = unpack2(chk[q]);
-      y = make_float2(y.x - z.y, y.y + z.x);
+    for (int q = 0; q < kOuts; ++q) {
+      if (c + q * cols >= count) continue;
+      float2 y = unpack2(acc[q]);
+      if constexpr (kCheck) {
+        const float2 z = unpack2(chk[q]);
+        y = make_float2(y.x - z.y, y.y + z.x);
+      }
+      L.out[m0 + c + q * cols] = y;
     }
-    L.out[m0 + l] = y;
-  }
+  };
+  if (L.per == kNatPer) run(std::integral_constant<int, kNatPer>());
+  else run(std::integral_constant<int, 1>());
 }
 
 // The history update alone (applies whose groups all ran on the tensor cores).
@@ -942,7 +946,7 @@ int PolyEngine::init(uint32_t fs, const fdsp_channel_cfg* ch, uint32_t nch, bool
     r = g0 % b;
     g0 = b;
   }
-  if (nch == 1 && !complex_taps && !chans_[0].nco.enabled && U0 >= (uint32_t)kNatMinUp && g0 == 1 && D0 <= 4u * U0 &&
+  if (nch == 1 && !complex_taps && !chans_[0].nco.enabled && U0 >= (uint32_t)kNatMinUp && U0 <= (uint32_t)kNatMaxCols && g0 == 1 && D0 <= 4u * U0 &&
       (uint64_t)U0 * chans_[0].T <= (uint64_t)kNatMaxTaps) {
     const uint32_t T0 = chans_[0].T;
     std::vector<float> host(((size_t)U0 * T0 + 3) & ~(size_t)3, 0.f);
@@ -1499,18 +1503,21 @@ int PolyEngine::launch_nat(const float2* d_in, uint64_t n, float2* out, bool che
   L.T = batches_[0].T;
   L.H = H_;
   // full tiles where they give every SM two, one output a thread otherwise
-  L.per = L.M >= 2LL * num_sms_ * kNatPer * kThreads ? kNatPer : 1;
-  const int64_t outs = (int64_t)L.per * kThreads;
+  L.cols = (int32_t)(k.up * std::max(1u, (uint32_t)kThreads / k.up));
+  if (L.cols < 192 && L.cols + (int32_t)k.up <= kNatMaxCols) L.cols += (int32_t)k.up;
+  L.per = L.M >= 2LL * num_sms_ * kNatPer * L.cols ? kNatPer : 1;
+  const int64_t outs = (int64_t)L.per * L.cols;
+  const int threads = (L.cols + 31) & ~31;
   L.len = (int32_t)((((outs - 1) * L.D + L.U - 1) / L.U + L.T + 1) & ~1LL);
   const size_t smem = (size_t)L.len * sizeof(float2) + (((size_t)L.U * L.T + 3) & ~(size_t)3) * sizeof(float);
   int tiles = (int)((L.M + outs - 1) / outs);
-  const int hist_blocks = (H_ + kThreads - 1) / kThreads;
+  const int hist_blocks = (H_ + threads - 1) / threads;
   const void* kern = check ? reinterpret_cast<const void*>(nat_resample_kernel<true>)
                            : reinterpret_cast<const void*>(nat_resample_kernel<false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_status(e);
   if (kprof_) cudaEventRecord(kprof_event(), stream);
-  e = klaunch(kern, dim3((unsigned)(tiles + hist_blocks)), dim3(kThreads), smem, stream, L, tiles);
+  e = klaunch(kern, dim3((unsigned)(tiles + hist_blocks)), dim3((unsigned)threads), smem, stream, L, tiles);
   if (kprof_) cudaEventRecord(kprof_event(), stream);
   if (e != cudaSuccess) return cuda_status(e);
   launches_last_++;

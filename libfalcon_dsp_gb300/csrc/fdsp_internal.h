@@ -125,7 +125,7 @@ struct NatLaunch {
   uint32_t phase;
   int32_t r_first;          // column of output 0
   int32_t U, D, T, H;
-  int32_t per;              // outputs a thread
+  int32_t cols, per;        // columns of a tile (a multiple of U, a thread each), outputs a thread
   int32_t len;              // samples a tile stages at most
 };
 
