@@ -32,17 +32,17 @@
 //               item's accumulator slot, commit frees the stage; the last
 //               chunk's commit hands the slot to the epilogue;
 //   warps 2-17  epilogue: four warps per TMEM lane quarter; each reads its
-//               (at most two) 8-slot column chunks out of tensor memory,
+//               (at most two) neighbouring 8-slot column chunks out of tensor memory,
 //               releases the slot, then rotates and stores;
-//   warp 18     scheduler: finds the CTA's next items (a warp-parallel
-//               cursor over the merge sets) and queues them for warp 0.
+//   warp 18     scheduler: queues the CTA's items for warp 0, from the list
+//               that the prep kernel sorted by first input sample.
 // Warps 0 and 1 run their loops in lane 0 alone.
 // Two accumulator slots of 256 columns (R tiles x N columns each) let the
 // MMAs of one item run while the epilogue drains the previous one.
 //
-// Each CTA owns a contiguous range of input samples and runs, in input
-// order, the items of every merge set that start in it, so the split input
-// is read from HBM about once and every group reuses it from L2.
+// The items of every merge set are listed in input order and cut into one run
+// of equal cost per CTA, so the split input is read from HBM about once and
+// every group reuses it from L2.
 //
 // Every mbarrier wait is bounded (TcLaunch::poll); a wait that runs out sets
 // the error flag (mapped host memory, read by fdsp_channelizer_status),
@@ -57,6 +57,7 @@
 #include <cstdint>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "fdsp_internal.h"
@@ -65,8 +66,7 @@
 
 namespace fdsp {
 
-constexpr int kTcEpiWarps = 16;                       // kTcEpiPerQ per TMEM lane quarter
-constexpr int kTcEpiPerQ = kTcEpiWarps / 4;
+constexpr int kTcEpiPerQ = kTcEpiWarps / 4;           // epilogue warps per TMEM lane quarter
 constexpr int kTcEpiOwn = 8 / kTcEpiPerQ;             // most column chunks a warp reads per item (R NS <= 64)
 constexpr int kTcSchedWarp = 2 + kTcEpiWarps;         // the item scheduler (after the epilogue warps)
 constexpr int kTcThreads = 96 + 32 * kTcEpiWarps;     // producer, MMA, epilogue and scheduler warps
@@ -146,69 +146,6 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
                : "memory");
 }
 
-// The sequence of items (merge set, item index) a CTA runs, walked by the
-// producer warp and announced to the MMA and epilogue warps through a ring of
-// (merge set, item) entries.  Items of merge set m start at input sample
-// a + t P; the next item is the earliest start (ties: the lower merge set).
-// Lane l keeps merge sets l and l + 32 in registers: its next start u, its
-// item range [cur, end) and P; a butterfly reduction picks the next item.
-struct TcCursor {
-  int64_t u[2], P[2];
-  int32_t cur[2], end[2];
-  __device__ void init(const TcMset* ms, const TcGroup* groups, int nmsets, int64_t Lc, int G, int b, int lane) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int m = lane + 32 * i;
-      cur[i] = end[i] = 0;
-      u[i] = P[i] = 0;
-      if (m >= nmsets) continue;
-      const TcMset& M = ms[m];
-      P[i] = (int64_t)M.R * kTcRows * groups[M.group].D;
-      int64_t f, l;
-      tc_item_range(M.a, P[i], M.items, Lc, b, G, &f, &l);
-      cur[i] = (int32_t)f;
-      end[i] = (int32_t)l;
-      u[i] = (int64_t)M.a + f * P[i];
-    }
-  }
-  // (whole warp; every lane returns the same item)
-  __device__ __forceinline__ bool next(int lane, int* m_out, int* t_out) {
-    int64_t bu = INT64_MAX;
-    int bm = INT32_MAX;
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-      if (cur[i] < end[i] && u[i] < bu) {
-        bu = u[i];
-        bm = lane + 32 * i;
-      }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const int64_t u2 = __shfl_xor_sync(0xffffffffu, bu, o);
-      const int m2 = __shfl_xor_sync(0xffffffffu, bm, o);
-      if (u2 < bu || (u2 == bu && m2 < bm)) {
-        bu = u2;
-        bm = m2;
-      }
-    }
-    if (bm == INT32_MAX) return false;
-    int t = 0;
-    if ((bm & 31) == lane) {
-      const int i = bm >> 5;
-      t = i ? cur[1] : cur[0];
-      if (i) {
-        cur[1]++;
-        u[1] += P[1];
-      } else {
-        cur[0]++;
-        u[0] += P[0];
-      }
-    }
-    *m_out = bm;
-    *t_out = __shfl_sync(0xffffffffu, t, bm & 31);
-    return true;
-  }
-};
-
 // Position in the stage ring: stage s of round r (chunk r * stages + s),
 // advanced without a division per chunk.
 struct TcRing {
@@ -221,8 +158,14 @@ struct TcRing {
   }
 };
 
+// Input samples between the starts of a merge set's items.
+__device__ __forceinline__ uint32_t tc_item_step(const TcMset& M, const TcGroup* groups) {
+  return (uint32_t)M.R * (uint32_t)kTcRows * (uint32_t)groups[M.group].D;
+}
+
 // ---------------------------------------------------------------------------
-// prep: split [history | block] into {hi, lo} parts and build the B images
+// prep: split [history | block] into {hi, lo} parts, build the B images and
+// the item list
 // ---------------------------------------------------------------------------
 // B image of merge set m, chunk c: N = 4 NS rows (columns of B) of 128
 // bytes, the 16-byte piece q of row n (taps 2q, 2q + 1 of the chunk) at
@@ -274,6 +217,29 @@ __global__ void __launch_bounds__(256) tc_prep_kernel(const __grid_constant__ Tc
       uint8_t* dst = L.bbuf + M.b + ((size_t)c * N + n) * 128 + (size_t)((q ^ (n & 7)) * 16);
       *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
     }
+    // the items in the order of their first input sample (ties: the lower
+    // merge set), each with the cost of all items before it: a division per
+    // merge set gives both
+    const int nitems = L.iprefix[L.nmsets];
+    for (int p = (int)blockIdx.x * 256 + (int)threadIdx.x; p < nitems; p += nb_build * 256) {
+      int m = 0, hi = L.nmsets;  // largest m with iprefix[m] <= p
+      while (hi - m > 1) {
+        const int mid = (m + hi) >> 1;
+        if (L.iprefix[mid] <= p) m = mid;
+        else hi = mid;
+      }
+      const int t = p - L.iprefix[m];
+      const uint32_t u = (uint32_t)L.ms[m].a + (uint32_t)t * tc_item_step(L.ms[m], L.groups);
+      uint32_t place = 0, cost = 0;
+      for (int k = 0; k < L.nmsets; ++k) {
+        // (items of k that start before this one; at the same sample the lower merge set goes first)
+        const uint32_t before = tc_items_before((uint32_t)L.ms[k].a, tc_item_step(L.ms[k], L.groups),
+                                                (uint32_t)L.ms[k].items, u + (k < m ? 1u : 0u));
+        place += before;
+        cost += before * tc_item_cost(L.ms[k]);
+      }
+      L.items[place] = make_uint2(((uint32_t)m << 26) | (uint32_t)t, cost);
+    }
     return;
   }
   const int64_t stride = (int64_t)(gridDim.x - nb_build) * 256;
@@ -308,14 +274,23 @@ struct TcEpiSlot {
   int64_t x0;     // NCO counter argument of row 0's window start (base + w0, unreduced)
   uint32_t R;     // counter rollover; 0: every output takes the exact path
   int32_t J;      // rows with an output
-  uint16_t U;     // output stride
-  uint16_t Tm1;   // taps - 1
-  uint32_t pair;  // 1: the next slot holds this channel's next output (one 16-byte store)
+  uint32_t stride;  // bytes from an output to the next row's
+  uint16_t flags;   // how its outputs are stored (TcSlot::flags the addresses allow)
+  uint16_t Tm1;     // taps - 1
 };
 static_assert(sizeof(TcEpiSlot) == kTcEpiSlotBytes, "epilogue slot table layout");
-static_assert(offsetof(TcEpiSlot, om) == 8 && offsetof(TcEpiSlot, R) == 32 && offsetof(TcEpiSlot, J) == 36 &&
-                  offsetof(TcEpiSlot, U) == 40 && offsetof(TcEpiSlot, Tm1) == 42 && offsetof(TcEpiSlot, pair) == 44,
-              "the epilogue reads a slot record as two 16-byte halves");
+static_assert(offsetof(TcEpiSlot, om) == 8 && offsetof(TcEpiSlot, fm) == 16 && offsetof(TcEpiSlot, x0) == 24 &&
+                  offsetof(TcEpiSlot, R) == 32 && offsetof(TcEpiSlot, J) == 36 && offsetof(TcEpiSlot, stride) == 40 &&
+                  offsetof(TcEpiSlot, flags) == 44 && offsetof(TcEpiSlot, Tm1) == 46,
+              "the epilogue reads a slot's table entry as three 16-byte parts");
+
+// What a warp needs of a slot for one block of 32 rows: made by one lane per
+// slot, read by every lane as 16-byte broadcasts.
+//   {address of the first row's output, row stride in bytes, scratch address}
+//   {counter of the first row, turns per sample (64 bits), -}
+//   {rollover, counters below this do not straddle it, rows (0-32), -}
+constexpr uint32_t kTcRec = 48;
+static_assert(kTcEpiRecs == 16 * (int)kTcRec && kTcEpiRows == 2048, "epilogue scratch: 32 rows x 8 outputs, 16 records");
 
 // Outputs whose window crosses the NCO rollover (or whose counter leaves the
 // fast path's 32-bit range) were stored unrotated; rotate_prep/rotate_apply
@@ -337,24 +312,32 @@ __device__ __noinline__ void tc_fix_exact(const TcLaunch& L, int slot, int64_t j
   float2 B = make_float2(0.f, 0.f);
   if (er.straddle) {
     const float2* g = L.ctaps[S.ch] + (size_t)S.phi * S.T;
-    for (int k = er.k0; k < (int)S.T; ++k) {
-      const float2 x = tc_load_x(L, w0 + k);
-      const float2 gk = __ldg(g + k);
-      B.x = fmaf(gk.x, x.x, B.x);
-      B.x = fmaf(-gk.y, x.y, B.x);
-      B.y = fmaf(gk.x, x.y, B.y);
-      B.y = fmaf(gk.y, x.x, B.y);
+    // eight taps' loads in flight at a time (one after another, each tap cost
+    // a memory latency); the sum runs in tap order
+    for (int k = er.k0; k < (int)S.T; k += 8) {
+      float2 x[8], gk[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int t = min(k + i, (int)S.T - 1);
+        x[i] = tc_load_x(L, w0 + t);
+        gk[i] = __ldg(g + t);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (k + i >= (int)S.T) break;
+        B.x = fmaf(gk[i].x, x[i].x, B.x);
+        B.x = fmaf(-gk[i].y, x[i].y, B.x);
+        B.y = fmaf(gk[i].x, x[i].y, B.y);
+        B.y = fmaf(gk[i].y, x[i].x, B.y);
+      }
     }
   }
   *dst = rotate_apply(er, *dst, B);
 }
 
-// Row stride D' of the merge set that holds slot s.
-__device__ __forceinline__ int64_t tc_slot_stride(const TcLaunch& L, int s) {
-  for (int m = 0; m < L.nmsets; ++m)
-    if (s >= L.ms[m].slot0 && s < L.ms[m].slot0 + L.ms[m].NS) return L.groups[L.ms[m].group].D;
-  return 0;
-}
+// Most rows of a slot (T taps, rows Dp samples apart) whose windows straddle
+// one rollover point.
+__host__ __device__ __forceinline__ int64_t tc_fix_rows(int64_t T, int64_t Dp) { return (T - 1 + Dp - 1) / Dp; }
 
 // Whether the filter-bank epilogue rotates slot S's rows itself (its fast
 // path); when not, every row of the slot was stored unrotated.
@@ -367,8 +350,10 @@ __device__ __forceinline__ bool tc_slot_fast(const TcLaunch& L, const NcoConst& 
 // window, so the product splits into the taps before and after it), or every
 // row of a slot whose rollover is too short (or too long) for the epilogue's
 // 32-bit counters.  Blocks (slot, y): the gridDim.y blocks of a slot take its
-// rollover points (or its rows) in turn.  Runs after the filter-bank launch
-// on the same stream.
+// rows in turn.  Runs after the filter-bank launch on the same stream.  Bound
+// by latency: a thread a rollover point, its rows one after another and a load
+// at a time, after a search for its merge set, took 27 us for 64 channels of
+// 4 M samples.
 __global__ void __launch_bounds__(128) tc_fix_kernel(const __grid_constant__ TcLaunch L) {
   const int s = blockIdx.x;
   if (s >= L.nslots) return;
@@ -376,8 +361,7 @@ __global__ void __launch_bounds__(128) tc_fix_kernel(const __grid_constant__ TcL
   if (S.J <= 0 || S.T == 0) return;
   const NcoConst nc = L.nco[S.ch];
   if (!nc.enabled || nc.omega64 == 0 || nc.rollover == 0) return;
-  const int64_t Dp = tc_slot_stride(L, s);
-  if (Dp <= 0) return;
+  const int64_t Dp = S.D;
   float2* out = reinterpret_cast<float2*>(S.out);
   const int64_t J = S.J, T = S.T, R = nc.rollover;
   const int64_t t0 = (int64_t)blockIdx.y * blockDim.x + threadIdx.x, tstep = (int64_t)gridDim.y * blockDim.x;
@@ -394,13 +378,13 @@ __global__ void __launch_bounds__(128) tc_fix_kernel(const __grid_constant__ TcL
   int64_t r0 = (base + first) % R;
   if (r0 < 0) r0 += R;
   const int64_t n0 = first + (r0 == 0 ? 0 : R - r0);
-  for (int64_t n = n0 + t0 * R; n <= last; n += tstep * R) {
-    // rows with n - T + 1 <= w0 + j D' <= n - 1
-    const int64_t lo = n - T + 1 - w0, hi = n - 1 - w0;
-    int64_t j0 = lo <= 0 ? 0 : (lo + Dp - 1) / Dp;
-    int64_t j1 = hi < 0 ? -1 : hi / Dp;
-    if (j1 > J - 1) j1 = J - 1;
-    for (int64_t j = j0; j <= j1; ++j) tc_fix_exact(L, s, j, Dp, out + (uint64_t)S.U * (uint64_t)j);
+  // a thread a row: at most tc_fix_rows rows straddle a point, those with
+  // n - T + 1 <= w0 + j D' <= n - 1
+  const int64_t per = tc_fix_rows(T, Dp), points = last < n0 ? 0 : (last - n0) / R + 1;
+  for (int64_t i = t0; i < points * per; i += tstep) {
+    const int64_t n = n0 + i / per * R, lo = n - T + 1 - w0;
+    const int64_t j = (lo <= 0 ? 0 : (lo + Dp - 1) / Dp) + i % per;
+    if (j < J && w0 + j * Dp <= n - 1) tc_fix_exact(L, s, j, Dp, out + (uint64_t)S.U * (uint64_t)j);
   }
 }
 
@@ -411,6 +395,18 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   return v;
 }
 
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void sts64(uint32_t addr, float2 v) {
+  asm volatile("st.shared.v2.f32 [%0], {%1, %2};\n" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
+}
+// 32-byte global store (32-byte aligned).
+__device__ __forceinline__ void stg256(void* p, const float2 (&o)[4]) {
+  asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(p), "f"(o[0].x), "f"(o[0].y),
+               "f"(o[1].x), "f"(o[1].y), "f"(o[2].x), "f"(o[2].y), "f"(o[3].x), "f"(o[3].y)
+               : "memory");
+}
 // ---------------------------------------------------------------------------
 // the filter-bank kernel
 // ---------------------------------------------------------------------------
@@ -462,17 +458,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_filter_kernel(const __grid_c
   for (int i = tid; i < L.ngroups; i += kTcThreads) s_groups[i] = L.groups[i];
   // epilogue constants of every slot of the launch (after the stages)
   TcEpiSlot* etab =
-      reinterpret_cast<TcEpiSlot*>(smem_raw + (sbase - tc::smem_u32(smem_raw)) + (size_t)stages * L.stage_bytes);
+      reinterpret_cast<TcEpiSlot*>(smem_raw + (sbase - tc::smem_u32(smem_raw)) + (size_t)L.table_off);
   for (int s = tid; s < L.nslots; s += kTcThreads) {
     const TcSlot& S = L.slots[s];
-    int64_t D = 2;
-    for (int m = 0; m < L.nmsets; ++m)
-      if (s >= L.ms[m].slot0 && s < L.ms[m].slot0 + L.ms[m].NS) D = L.groups[L.ms[m].group].D;
+    const int64_t D = S.D;
     TcEpiSlot e;
     e.out = S.out;
     e.J = S.J;
-    e.U = S.U;
-    e.pair = S.flags & 1u;
+    e.stride = 8u * S.U;
+    // runs leave in 16-byte pieces from their first output, pairs and quads
+    // are single stores (rows 32 apart keep the alignment)
+    const uint64_t lo = e.out | e.stride;
+    uint32_t flags = S.flags;
+    if (((e.out - 8u * (uint32_t)tc_run_pos((int)flags)) & 15u) != 0u) flags &= ~(uint32_t)kTcRun;
+    if ((flags & kTcRun) || (lo & 15u) != 0u) flags &= ~(uint32_t)kTcPair;
+    if ((lo & 31u) != 0u) flags &= ~(uint32_t)kTcQuad;
+    e.flags = (uint16_t)flags;
     e.Tm1 = (uint16_t)(S.T > 0 ? S.T - 1u : 0u);
     e.om = 0;
     e.fm = 0;
@@ -570,33 +571,57 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_filter_kernel(const __grid_c
     }
   } else if (warp == kTcSchedWarp) {
     // ------------------------------------------------------------ scheduler
-    // The CTA's item sequence (warp-parallel cursor), kTcQueue items ahead of
-    // the producer; an item with merge set -1 ends it.
-    TcCursor cur;
-    cur.init(s_ms, s_groups, L.nmsets, L.Lc, L.G, blockIdx.x, lane);
-    bool failed = false;
-    for (int i = 0; !hold; ++i) {
-      int m = -1, t = 0;
-      const bool more = cur.next(lane, &m, &t);
+    // The CTA's part of the item list, up to 32 items a round, into the
+    // producer's queue; an item with merge set -1 ends it.  The list is cut by
+    // cost, not by input range: with few, uneven items (64 channels of 4 M
+    // samples: 17 an SM of 4 to 65 chunks) equal ranges left the slowest SM
+    // 2.5 times the average work.
+    const int nitems = L.iprefix[L.nmsets];
+    // first item whose cost before it is at least lim
+    auto lower = [&](uint32_t lim) {
+      int lo = 0, hi = nitems;  // 32 probes a round
+      while (hi > lo) {
+        const int step = (hi - lo + 32) / 33, p = lo + step * (lane + 1) - 1;
+        const bool less = p < hi && __ldg(&L.items[p].y) < lim;
+        const int n = __popc(__ballot_sync(0xffffffffu, less));  // (costs only grow along the list)
+        const int nlo = lo + step * n;
+        if (n < 32) hi = min(hi, nlo + step - 1);  // (probe n is not less)
+        lo = min(nlo, hi);
+      }
+      return lo;
+    };
+    const uint32_t end = tc_cost_bound(L.ctotal, (int)blockIdx.x + 1, L.G);  // the items before this cost are ours
+    const int first = lower(tc_cost_bound(L.ctotal, (int)blockIdx.x, L.G));
+    bool failed = false, more = !hold;
+    for (int done = 0; more;) {
+      const int at = first + done + lane;
+      const uint2 v = at < nitems ? __ldg(&L.items[at]) : make_uint2(0u, 0xFFFFFFFFu);
+      int room = 0;
       if (lane == 0) {
         uint32_t polls = 0;
-        while (i - *reinterpret_cast<volatile int*>(&q_cons) >= kTcQueue) {  // room in the queue
+        while ((room = kTcQueue - (done - *reinterpret_cast<volatile int*>(&q_cons))) <= 0) {
           if (++polls > poll) {
             failed = true;
             break;
           }
           __nanosleep(64);
         }
-        if (!failed) {
-          volatile int* qi = reinterpret_cast<volatile int*>(&q_items[i % kTcQueue]);
-          qi[0] = more ? m : -1;
-          qi[1] = more ? t : 0;
-          __threadfence_block();
-          *reinterpret_cast<volatile int*>(&q_prod) = i + 1;
-        }
       }
       failed = __shfl_sync(0xffffffffu, failed ? 1 : 0, 0) != 0;
-      if (!more || failed) break;
+      if (failed) break;
+      const bool item = v.y < end;
+      const int count = __popc(__ballot_sync(0xffffffffu, item));  // (a run from lane 0 on: costs grow)
+      const int n = min(min(__shfl_sync(0xffffffffu, room, 0), 32), count + 1);
+      if (lane < n) {
+        volatile int* qi = reinterpret_cast<volatile int*>(&q_items[(done + lane) % kTcQueue]);
+        qi[0] = item ? (int)(v.x >> 26) : -1;
+        qi[1] = (int)(v.x & 0x3FFFFFFu);
+      }
+      more = n <= count;  // the end marker is not yet among them
+      __threadfence_block();  // the items are written before the count
+      __syncwarp();
+      done += n;
+      if (lane == 0) *reinterpret_cast<volatile int*>(&q_prod) = done;
     }
     if (failed && lane == 0) atomicExch(L.err, 1);
   } else if (warp == 1) {
@@ -664,9 +689,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_filter_kernel(const __grid_c
     }
   } else {
     // ------------------------------------------------------------ epilogue
+    // It used to bound the kernel: 16 warps took ~9000 cycles an item (87
+    // instructions per 32 outputs at one in 6 cycles a warp), while the
+    // accumulator waited for them.  So one lane per slot prepares what a block
+    // of 32 rows needs, and a block whose rows all exist and whose counters do
+    // not roll over (all but a few in a hundred) runs without a test per
+    // output; its stores are chosen by warp-uniform masks.  Rows of 3, 5, 6 or
+    // 7 outputs go through shared memory and leave in whole lines, rows of a
+    // multiple of 4 as 32-byte stores: the sectors written fell from 2.5 times
+    // the outputs to 1.1 times.  The 256-channel step of 2^26 samples went from
+    // 5.14 to 4.83 ms, 64 taps over 2^24 samples from 156 to 140 us; the MMA
+    // side now sets the pace (~7000 cycles an item: 12 KB of operands read and
+    // 12 KB filled per MMA are 192 cycles of shared memory for 128 of tensor
+    // work).  Nothing here may spill: with the stages in shared memory the L1
+    // is too small, and 20 spilled registers doubled the kernel's time.
     const int q = warp & 3;           // TMEM lane quarter this warp may read
-    const int h = (warp - 2) >> 2;    // which of the item's column chunks (every kTcEpiPerQ-th)
+    const int h = (warp - 2) >> 2;    // which of the item's column chunks
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
+    const uint32_t etab_s = tc::smem_u32(etab);
+    const uint32_t scr = sbase + (uint32_t)L.scratch_off + (uint32_t)(warp - 2) * (uint32_t)L.scratch_warp;  // 32 rows x 8 outputs (where the launch has runs)
+    const uint32_t rec = scr + (uint32_t)L.scratch_warp - 16u * kTcRec;  // a record per slot
     bool failed = false;
     for (int k = 0;; ++k) {
       const int a = k & 1;
@@ -682,20 +724,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_filter_kernel(const __grid_c
       const int m = it.x, t = it.y;
       const TcMset& M = s_ms[m];
       const int R = M.R, NS = M.NS, nch = NS >> 3;
-      const int64_t D = s_groups[M.group].D;
-      const uint32_t laneD = (uint32_t)lane * (uint32_t)D;
-      // every column chunk this warp owns (at most kTcEpiOwn: R * NS <= 64)
-      // is read out of tensor memory first and the accumulator slot
-      // released, so the MMAs of a later item run while this warp rotates
+      const int D = s_groups[M.group].D;
+      // the warp's column chunks (8 slots of a tile each, at most kTcEpiOwn:
+      // R NS <= 64) are read out of tensor memory together and the accumulator
+      // slot released, so the MMAs of a later item run while this warp rotates
       // and stores
-      const int n_own = (R * nch - h + kTcEpiPerQ - 1) / kTcEpiPerQ;  // chunks h, h + kTcEpiPerQ, ...
-      float yv[kTcEpiOwn][16];                                       // (hi + lo) sums of those chunks
+      const int per = (R * nch + kTcEpiPerQ - 1) / kTcEpiPerQ;  // 1 or 2
+      const int idx0 = h * per, n_own = min(per, R * nch - idx0);
+      float yv[kTcEpiOwn][16];  // (hi + lo) sums of those chunks
 #pragma unroll
       for (int u = 0; u < kTcEpiOwn; ++u) {
         if (u < n_own) {
-          const int idx = h + kTcEpiPerQ * u;
-          const int r = idx / nch, cc = idx - r * nch;
-          const uint32_t col = tbase + lane_off + (uint32_t)a * 256u + (uint32_t)(r * (256 / R) + 16 * cc);
+          const int idx = idx0 + u, r = idx >= nch ? 1 : 0, cc = idx - r * nch;
+          const uint32_t col = tbase + lane_off + (uint32_t)a * 256u + (uint32_t)(r * 128 + 16 * cc);
           uint32_t vh[16], vl[16];
           tc::tmem_ld16(col, vh);
           tc::tmem_ld16(col + (uint32_t)(2 * NS), vl);
@@ -707,76 +748,150 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_filter_kernel(const __grid_c
       tc::fence_before_sync();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&acc_empty[a]);
-      // one copy of the chunk code (kept small: the warps of every role share
-      // the SM's instruction cache); the chunks move down into yv[0] in turn
+      // the records: lane e makes the one of slot e & 7 of chunk e >> 3
+      uint32_t rows = 0, flags = 0;
+      bool plain = true;   // every row or none, no rollover in any window of the block
+      bool first = false;  // the first slot of a run
+      if ((lane >> 3) < n_own) {
+        const int idx = idx0 + (lane >> 3), r = idx >= nch ? 1 : 0, cc = idx - r * nch;
+        const int row0 = (t * R + r) * kTcRows + q * 32;  // row of lane 0
+        const uint32_t e = etab_s + (uint32_t)(M.slot0 + cc * 8 + (lane & 7)) * kTcEpiSlotBytes;
+        const uint4 ea = lds128(e), eb = lds128(e + 16u), ec = lds128(e + 32u);
+        const uint64_t out = (uint64_t)ea.x | ((uint64_t)ea.y << 32);
+        const uint32_t Rr = ec.x, Tm1 = ec.w >> 16;
+        rows = (uint32_t)min(max((int)ec.y - row0, 0), 32);
+        const uint64_t ptr = out + (uint64_t)ec.z * (uint64_t)(uint32_t)row0;
+        // NCO counter of the first row's window start, (x0 + row0 D) mod R:
+        // 0 <= x0 + row0 D < 2^32 or > -R on the fast path
+        uint32_t p0 = 0, lim = 0xFFFFFFFFu, Rc = 0xFFFFFFFFu;
+        if ((ea.z | ea.w) != 0u) {
+          const int64_t v = (int64_t)((uint64_t)eb.z | ((uint64_t)eb.w << 32)) + (int64_t)row0 * D;
+          const uint64_t fm = (uint64_t)eb.x | ((uint64_t)eb.y << 32);
+          Rc = Rr;
+          lim = Rr > Tm1 ? Rr - Tm1 : 0u;  // (R = 0: every row of the slot is left to tc_fix_kernel)
+          if (Rr != 0u)
+            p0 = v < 0 ? (uint32_t)(v + (int64_t)Rr) : (uint32_t)__umul64hi(fm * (uint64_t)(uint32_t)v, (uint64_t)Rr);
+        }
+        plain = rows == 0u || (rows == 32u && (uint64_t)p0 + 31u * (uint32_t)D < (uint64_t)lim);
+        flags = ec.w & 0xFFFFu;
+        const uint32_t pos = (uint32_t)tc_run_pos((int)flags);
+        const uint32_t ra = rec + (uint32_t)lane * kTcRec;
+        sts128(ra, (uint32_t)ptr, (uint32_t)(ptr >> 32), ec.z, scr + (uint32_t)(lane & 7) * 256u - pos * 248u);
+        sts128(ra + 16u, p0, ea.z, ea.w, 0u);
+        sts128(ra + 32u, Rc, lim, rows, 0u);
+        first = (flags & kTcRun) != 0u && pos == 0u;
+      }
+      const uint32_t m_plain = __ballot_sync(0xffffffffu, plain);
+      const uint32_t m_live = __ballot_sync(0xffffffffu, rows > 0u);
+      const uint32_t m_run = __ballot_sync(0xffffffffu, (flags & kTcRun) != 0u);
+      const uint32_t m_first = __ballot_sync(0xffffffffu, first);
+      const uint32_t m_pair = __ballot_sync(0xffffffffu, (flags & kTcPair) != 0u);
+      const uint32_t m_quad = __ballot_sync(0xffffffffu, (flags & kTcQuad) != 0u);
+      const uint32_t laneD = (uint32_t)lane * (uint32_t)D;
+      // one chunk of 8 slots; kPlain: every lane has its row and no counter
+      // rolls over (else both are tested per output)
+      auto chunk = [&](int u, auto plain_tag) {
+        constexpr bool kPlain = decltype(plain_tag)::value;
+        const uint32_t rc = rec + (uint32_t)u * 8u * kTcRec;
+        const uint32_t live = m_live >> (8 * u), run = m_run >> (8 * u), pair = m_pair >> (8 * u),
+                       quad = m_quad >> (8 * u);
+#pragma unroll
+        for (int g = 0; g < 8; g += 4) {  // four slots at a time
+          if (((live >> g) & 15u) == 0u) continue;  // padding slots: nothing to do
+          float2 o[4];
+          bool v[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const uint4 rb = lds128(rc + (uint32_t)(g + e) * kTcRec + 16u);
+            const float2 y0 = make_float2(yv[0][2 * (g + e)], yv[0][2 * (g + e) + 1]);
+            uint32_t pc = rb.x + laneD;
+            bool fast = true;
+            v[e] = true;
+            if constexpr (!kPlain) {
+              const uint4 rr = lds128(rc + (uint32_t)(g + e) * kTcRec + 32u);
+              pc = pc >= rr.x ? pc - rr.x : pc;
+              fast = pc < rr.y;
+              v[e] = (uint32_t)lane < rr.z;
+            }
+            const uint32_t turns = __umulhi(pc, rb.y) + pc * rb.z;  // bits 32..63 of pc * om: 2^-32 turns
+            float sn, cs;
+            __sincosf((float)(int32_t)turns * 1.4629180792671596e-09f, &sn, &cs);  // 2 pi / 2^32
+            o[e] = cmul_nco(y0, make_float2(cs, sn));
+            if constexpr (!kPlain) o[e] = fast ? o[e] : y0;  // windows across the rollover: unrotated, for tc_fix_kernel
+          }
+          auto dst = [&](int e) {
+            const uint4 r0 = lds128(rc + (uint32_t)(g + e) * kTcRec);
+            return reinterpret_cast<float2*>(((uint64_t)r0.x | ((uint64_t)r0.y << 32)) +
+                                             (uint64_t)r0.z * (uint64_t)(uint32_t)lane);
+          };
+          if ((quad >> g) & 1u) {
+            if (v[3]) {
+              stg256(dst(0), o);
+              continue;
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) {
+            if ((pair >> (g + e)) & 1u) {
+              if (v[e + 1])
+                __stcs(reinterpret_cast<float4*>(dst(e)), make_float4(o[e].x, o[e].y, o[e + 1].x, o[e + 1].y));
+              else if (v[e])
+                __stcs(dst(e), o[e]);
+              continue;
+            }
+#pragma unroll
+            for (int f = e; f < e + 2; ++f) {
+              if ((run >> (g + f)) & 1u) {  // rows of the run follow one another in the scratch
+                const uint4 r0 = lds128(rc + (uint32_t)(g + f) * kTcRec);
+                if (v[f]) sts64(r0.w + r0.z * (uint32_t)lane, o[f]);
+              } else if ((live >> (g + f)) & 1u) {
+                if (v[f]) __stcs(dst(f), o[f]);
+              }
+            }
+          }
+        }
+      };
+      // one copy of the chunk code of either kind (kept small: the warps of
+      // every role share the SM's instruction cache); the chunks move down
+      // into yv[0] in turn
 #pragma unroll 1
       for (int u = 0; u < n_own; ++u) {
         if (u > 0) {
 #pragma unroll
-          for (int w = 0; w + 1 < kTcEpiOwn; ++w)
-#pragma unroll
-            for (int i = 0; i < 16; ++i) yv[w][i] = yv[w + 1][i];
+          for (int i = 0; i < 16; ++i) yv[0][i] = yv[1][i];
         }
-        const int idx = h + kTcEpiPerQ * u;
-        const int r = idx / nch, cc = idx - r * nch;
-        const int64_t row0 = ((int64_t)t * R + r) * kTcRows + q * 32;  // row of lane 0
-        const int64_t j = row0 + lane;
-        const TcEpiSlot* E8 = etab + M.slot0 + cc * 8;
-        // NCO counter of lane 0's window start for slot e (lane e computes it):
-        // (x0 + row0 D) mod R, once per chunk; 0 <= x0 + row0 D < 2^32 or
-        // > -R on the fast path
-        uint32_t p0 = 0;
-        if (lane < 8) {
-          const TcEpiSlot& E = E8[lane];
-          if (E.om != 0 && E.R != 0) {
-            const int64_t v = E.x0 + row0 * D;
-            p0 = v < 0 ? (uint32_t)(v + (int64_t)E.R)
-                       : (uint32_t)__umul64hi(E.fm * (uint64_t)(uint32_t)v, (uint64_t)E.R);
-          }
-        }
-        // per pair of slots: their constants as two 16-byte shared loads each
-        // ({out, om} and {R, J, U | Tm1 << 16, pair}), the rotation, and one
-        // 16-byte store where a slot and the next hold the same channel's
-        // consecutive outputs (contiguous across the lanes when the outputs
-        // interleave by two)
-        const uint32_t e8 = tc::smem_u32(E8);
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-          const uint4 b0 = lds128(e8 + (uint32_t)e * kTcEpiSlotBytes + 32u);
-          const uint4 b1 = lds128(e8 + (uint32_t)(e + 1) * kTcEpiSlotBytes + 32u);
-          if ((int32_t)b0.y <= 0 && (int32_t)b1.y <= 0) continue;  // two padding slots (no rows): nothing to do
-          const uint4 a0 = lds128(e8 + (uint32_t)e * kTcEpiSlotBytes);
-          const uint4 a1 = lds128(e8 + (uint32_t)(e + 1) * kTcEpiSlotBytes);
-          float2 o[2];
-#pragma unroll
-          for (int k2 = 0; k2 < 2; ++k2) {
-            const uint4 A = k2 ? a1 : a0, Bv = k2 ? b1 : b0;
-            const uint32_t Rr = Bv.x, Tm1 = Bv.z >> 16, om_lo = A.z, om_hi = A.w;
-            const uint32_t P0 = __shfl_sync(0xffffffffu, p0, e + k2);
-            const float2 y0 = make_float2(yv[0][2 * (e + k2)], yv[0][2 * (e + k2) + 1]);
-            uint32_t pc = P0 + laneD;
-            pc = pc >= Rr ? pc - Rr : pc;
-            const bool fast = pc + Tm1 < Rr || (om_lo | om_hi) == 0u;
-            const uint32_t turns = __umulhi(pc, om_lo) + pc * om_hi;  // bits 32..63 of pc * om: 2^-32 turns
-            float sn, cs;
-            __sincosf((float)(int32_t)turns * 1.4629180792671596e-09f, &sn, &cs);  // 2 pi / 2^32
-            const float2 y = cmul_nco(y0, make_float2(cs, sn));
-            o[k2] = fast ? y : y0;  // windows across the NCO rollover: unrotated, for tc_fix_kernel
-          }
-          float2* d0 = reinterpret_cast<float2*>((uint64_t)a0.x | ((uint64_t)a0.y << 32)) +
-                       (uint64_t)(b0.z & 0xFFFFu) * (uint64_t)j;
-          const bool v0 = j < (int64_t)(int32_t)b0.y, v1 = j < (int64_t)(int32_t)b1.y;
-          if (b0.w != 0u && v0 && v1 && (reinterpret_cast<uintptr_t>(d0) & 15u) == 0) {
-            __stcs(reinterpret_cast<float4*>(d0), make_float4(o[0].x, o[0].y, o[1].x, o[1].y));
-          } else {
-            if (v0) __stcs(d0, o[0]);
-            if (v1)
-              __stcs(reinterpret_cast<float2*>((uint64_t)a1.x | ((uint64_t)a1.y << 32)) +
-                         (uint64_t)(b1.z & 0xFFFFu) * (uint64_t)j,
-                     o[1]);
-          }
+        __syncwarp();  // the records; the scratch rows of the last chunk are read
+        if (((m_plain >> (8 * u)) & 255u) == 255u)
+          chunk(u, std::true_type());
+        else
+          chunk(u, std::false_type());
+        // complete runs leave in whole lines: 32 rows of len outputs follow one
+        // another in the scratch as they do in the channel's output
+        uint32_t firsts = (m_first >> (8 * u)) & 255u;
+        if (firsts != 0u) {
+          __syncwarp();
+          do {
+            const uint32_t e = (uint32_t)__ffs((int)firsts) - 1u, ra = rec + (8u * (uint32_t)u + e) * kTcRec;
+            firsts &= firsts - 1u;
+            const uint4 r0 = lds128(ra);
+            const uint64_t ptr = (uint64_t)r0.x | ((uint64_t)r0.y << 32);
+            const uint32_t len = r0.z >> 3, src = scr + e * 256u;
+            if (lds128(ra + (len - 1u) * kTcRec + 32u).z == 32u) {
+              for (uint32_t i = (uint32_t)lane; i < 16u * len; i += 32u)
+                __stcs(reinterpret_cast<uint4*>(ptr) + i, lds128(src + 16u * i));
+            } else {  // the last rows of the channel
+              uint32_t count = 0;
+              for (uint32_t f = 0; f < len; ++f) count += lds128(ra + f * kTcRec + 32u).z;
+              for (uint32_t i = (uint32_t)lane; i < count; i += 32u) {
+                float2 w;
+                asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];\n" : "=f"(w.x), "=f"(w.y) : "r"(src + 8u * i));
+                __stcs(reinterpret_cast<float2*>(ptr) + i, w);
+              }
+            }
+          } while (firsts != 0u);
         }
       }
+      __syncwarp();  // the records are read before the next item's are made
     }
     if (failed && lane == 0) atomicExch(L.err, 1);
   }
@@ -812,6 +927,7 @@ void PolyEngine::free_tc() {
   if (d_ctab_) dfree(d_ctab_);
   if (d_xhl_) dfree(d_xhl_);
   if (d_bbuf_) dfree(d_bbuf_);
+  if (d_items_) dfree(d_items_);
   if (d_tcrec_) dfree(d_tcrec_);
   for (cudaEvent_t e : pack_ev_) cudaEventDestroy(e);
   pack_ev_.clear();
@@ -822,6 +938,8 @@ void PolyEngine::free_tc() {
   d_ctab_ = nullptr;
   d_xhl_ = nullptr;
   d_bbuf_ = nullptr;
+  d_items_ = nullptr;
+  items_cap_ = 0;
   d_tcrec_ = nullptr;
   h_err_ = nullptr;
   d_err_ = nullptr;
@@ -990,8 +1108,11 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
   // images of every pack (a 1 KB aligned region each)
   int64_t xhl_need = 0;
   size_t b_need = 0;
-  std::vector<size_t> boff(plans.size());
+  std::vector<size_t> boff(plans.size()), ioff(plans.size());
+  size_t i_need = 0;
   for (size_t li = 0; li < plans.size(); ++li) {
+    ioff[li] = i_need;
+    i_need += (size_t)plans[li].items;
     xhl_need = std::max(xhl_need, plans[li].xhl_samples);
     boff[li] = b_need;
     b_need += (plans[li].b_bytes + 1023u) & ~(size_t)1023u;
@@ -1009,6 +1130,13 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
     bbuf_cap_ = 0;
     FDSP_TRY(cuda_status(dalloc(reinterpret_cast<void**>(&d_bbuf_), b_need)));
     bbuf_cap_ = b_need;
+  }
+  if (i_need > items_cap_) {
+    if (d_items_) dfree(d_items_);
+    d_items_ = nullptr;
+    items_cap_ = 0;
+    FDSP_TRY(cuda_status(dalloc(reinterpret_cast<void**>(&d_items_), i_need * sizeof(uint2))));
+    items_cap_ = i_need;
   }
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) return FDSP_ERR_UNSUPPORTED;
@@ -1047,6 +1175,9 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
     L.ngroups = (int32_t)plan.groups.size();
     L.stages = plan.stages;
     L.stage_bytes = plan.stage_bytes;
+    L.table_off = plan.table_off;
+    L.scratch_off = plan.scratch_off;
+    L.scratch_warp = plan.scratch_warp;
     L.nslots = (int32_t)plan.slots.size();
     L.poll = tc_poll_;
     L.hold = tc_hold_;
@@ -1062,6 +1193,14 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
       pieces += plan.ms[m].nchunks * 4 * plan.ms[m].NS * 8;
     }
     L.bprefix[plan.ms.size()] = pieces;
+    L.items = d_items_ + ioff[li];
+    int items = 0;
+    for (size_t m = 0; m < plan.ms.size(); ++m) {
+      L.iprefix[m] = items;
+      items += plan.ms[m].items;
+    }
+    L.iprefix[plan.ms.size()] = items;
+    for (const TcMset& m : plan.ms) L.ctotal += (uint32_t)m.items * tc_item_cost(m);
     for (size_t s = 0; s < plan.slots.size(); ++s) {
       L.slots[s] = plan.slots[s];
       if (plan.slots[s].J > 0)
@@ -1085,7 +1224,7 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
       if (r != CUDA_SUCCESS) return FDSP_ERR_UNSUPPORTED;
     }
     // prep: B images (few blocks), then, for the first launch, the split
-    const int nb_build = std::max(1, std::min(num_sms_, (pieces + 255) / 256));
+    const int nb_build = std::max(1, std::min(num_sms_, (std::max(pieces, items) + 255) / 256));
     const int64_t nb_split = li == 0 ? std::min<int64_t>((xhl_need + 255) / 256, (int64_t)num_sms_ * 8) : 0;
     auto prep = tc_fmt_ == 0 ? tc_prep_kernel<0> : tc_prep_kernel<1>;
     int nbb = nb_build;
@@ -1106,21 +1245,19 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
     if (kprof_) cudaEventRecord(kprof_event(), ps);
     if (e != cudaSuccess) return cuda_status(e);
     launches_last_++;
-    // exact pass: blocks per slot for the most rows (or rollover points) a
-    // slot of this launch has to fix, one per thread (the pass is latency
-    // bound: each point is a serial T-tap sum, and the last pack's pass ends
-    // the step)
+    // exact pass: blocks per slot for the most rows a slot of this launch may
+    // have to fix, one per thread (the pass is latency bound: each row is a
+    // serial sum of up to T taps, and the last pack's pass ends the step)
     int64_t work = 1;
     for (size_t si = 0; si < plan.slots.size(); ++si) {
       const TcSlot& S = plan.slots[si];
       if (S.J <= 0) continue;
       const NcoConst& nc = chans_[S.ch].nco;
       if (!nc.enabled || nc.omega64 == 0 || nc.rollover == 0) continue;
-      int64_t Dp = 0;
-      for (const TcMset& m : plan.ms)
-        if ((int)si >= m.slot0 && (int)si < m.slot0 + m.NS) Dp = plan.groups[m.group].D;
+      const int64_t Dp = S.D;
       const bool fast = !tc_exact_all_ && nc.rollover < 0x80000000u && 31 * Dp + S.T < (int64_t)nc.rollover;
-      work = std::max<int64_t>(work, fast ? ((int64_t)S.J * Dp + S.T) / nc.rollover + 1 : (int64_t)S.J);
+      work = std::max<int64_t>(
+          work, fast ? (((int64_t)S.J * Dp + S.T) / nc.rollover + 1) * tc_fix_rows(S.T, Dp) : (int64_t)S.J);
     }
     const unsigned fix_y = (unsigned)std::min<int64_t>(4096, (work + 127) / 128);
     e = klaunch(reinterpret_cast<const void*>(tc_fix_kernel), dim3((unsigned)plan.slots.size(), fix_y), dim3(128), 0,

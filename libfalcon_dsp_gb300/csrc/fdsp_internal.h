@@ -151,10 +151,16 @@ struct TcLaunch {
   int64_t Lc;                        // samples of the time range each CTA owns
   int64_t xhl_n;                     // samples of xhl the prep writes
   int32_t H, G, nmsets, ngroups, stages, stage_bytes, nslots;
+  int32_t table_off, scratch_off;    // epilogue slot table and warps' scratch in shared memory
   uint32_t poll;                     // polls before a wait gives up (each suspends up to ~2 us)
   int32_t hold;                      // test hook: the producer issues nothing (every wait runs out)
   int32_t exact_all;                 // test hook: every output takes the exact rotation pass
   int32_t bprefix[kTcMaxMsets + 1];  // 16-byte pieces of the B images before merge set m
+  int32_t iprefix[kTcMaxMsets + 1];  // items before merge set m
+  uint2* items;                      // every item by first input sample: {merge set << 26 | item, cost before it} (prep writes it)
+  uint32_t ctotal;                   // cost of all items
+  int32_t scratch_warp;              // scratch bytes of an epilogue warp: rows of runs (if any), then records
+  uint32_t pad_[2];
   TcGroup groups[kTcMaxGroups];
   TcMset ms[kTcMaxMsets];
   TcSlot slots[kTcMaxSlots];
@@ -387,6 +393,8 @@ class PolyEngine {
   std::vector<cudaStream_t> side_;     // launch packs 1.. (beside pack 0 on the caller's stream)
   std::vector<cudaEvent_t> pack_ev_;   // [0]: the split is done; [1 + i]: side stream i joins
   size_t bbuf_cap_ = 0;
+  uint2* d_items_ = nullptr;           // scratch: sorted items of the current apply (a region per launch pack)
+  size_t items_cap_ = 0;
   int* h_err_ = nullptr;               // bounded-wait failures, mapped host memory
   int* d_err_ = nullptr;               // its device address
   uint32_t tc_poll_ = 1u << 20;

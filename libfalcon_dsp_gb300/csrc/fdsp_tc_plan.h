@@ -56,6 +56,9 @@ constexpr int kTcStageMaxBytes = 49152;
 constexpr int kTcSmemDyn = 223 * 1024; // dynamic shared memory ceiling (227 KB minus static and alignment)
 constexpr int kTcMaxStages = 6;
 constexpr int kTcEpiSlotBytes = 48;    // per-slot epilogue constants staged in shared memory
+constexpr int kTcEpiWarps = 16;        // epilogue warps, each with its own scratch:
+constexpr int kTcEpiRows = 32 * 8 * 8; // 32 rows of 8 outputs (launches with runs)
+constexpr int kTcEpiRecs = 16 * 48;    // and a record per slot of two chunks
 
 // ---- launch records (kernel parameters; shared with the device code) -----
 struct TcGroup {
@@ -81,9 +84,19 @@ struct TcSlot {
   uint16_t U;       // output stride (up rate x row split)
   uint16_t o;       // window start inside the merge set's window (taps)
   uint16_t phi;     // tap phase
-  uint16_t flags;   // bit 0: the next slot holds the same channel's next output (pair store)
-  uint16_t pad_[2];
+  uint16_t flags;   // kTcPair .. kTcRun
+  uint16_t D;       // row stride D' (samples)
+  uint16_t pad_;
 };
+
+// Slot flags: how the epilogue stores a slot's outputs (8 slots, a column
+// chunk, are one warp's).
+constexpr int kTcPair = 1;      // the next slot holds the same channel's next output (16-byte store)
+constexpr int kTcQuad = 2;      // and the two after it, rows multiples of 32 bytes (32-byte store)
+constexpr int kTcRun = 4;       // one of a row's outputs, all of them in this chunk: bits 4-7 their number (3-8),
+                                // bits 8-11 this one's place (rows follow one another without gaps)
+FDSP_HD constexpr int tc_run_len(int flags) { return (flags >> 4) & 15; }
+FDSP_HD constexpr int tc_run_pos(int flags) { return (flags >> 8) & 15; }
 static_assert(sizeof(TcSlot) == 32, "slot record");
 static_assert(sizeof(TcMset) == 32, "merge-set record");
 
@@ -111,7 +124,9 @@ struct TcPlan {
   std::vector<int> slot_r;        // output offset r of each slot (for the out pointer)
   size_t b_bytes = 0;
   int64_t xhl_samples = 0;        // [history | block | zero pad] samples the split writes
-  int stages = 0, stage_bytes = 0, smem = 0;  // smem: stages, then the epilogue slot table
+  int stages = 0, stage_bytes = 0, smem = 0;  // smem: stages, the epilogue slot table, the epilogue warps' scratch
+  int table_off = 0, scratch_off = 0;         // (from the 1 KB aligned start)
+  int scratch_warp = 0;                       // bytes of a warp's scratch
   int G = 0;                      // grid (CTAs)
   int64_t Lc = 0;                 // samples of the time range each CTA owns
   int64_t items = 0;
@@ -269,6 +284,49 @@ inline int tc_choose_split(const std::vector<TcSlotIn>& xs, int D, int max_split
   return bestS;
 }
 
+// Positions of bundles [i, j) in a merge set of NS slots.  The epilogue's warps
+// take 8 slots each, so bundles are packed into runs of 8 where they fit
+// (widest first, first fit: 6 + 2, 3 + 3 + 1 + 1, 4 + 4), which keeps a row's
+// outputs in one warp; where that would need more columns they sit back to
+// back.  Position b of `order` starts at at[b].
+inline void tc_arrange(const std::vector<TcBundle>& bs, size_t i, size_t j, int NS, std::vector<int>& order,
+                       std::vector<int>& at) {
+  order.clear();
+  at.clear();
+  for (size_t b = i; b < j; ++b) order.push_back((int)b);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return bs[a].width > bs[b].width; });
+  int used[kTcMsetSlots / 8] = {0};
+  const int bins = NS / 8;
+  bool fits = true;
+  for (int b : order) {
+    const int w = bs[b].width, whole = w / 8, rest = w % 8;
+    int p = -1;
+    for (int c = 0; c + whole + (rest ? 1 : 0) <= bins && p < 0; ++c) {
+      if (whole == 0) {
+        if (used[c] + rest <= 8) p = c * 8 + used[c];
+        continue;
+      }
+      bool free = true;
+      for (int k = 0; k < whole + (rest ? 1 : 0); ++k) free = free && used[c + k] == 0;
+      if (free) p = c * 8;
+    }
+    if (p < 0) {
+      fits = false;
+      break;
+    }
+    at.push_back(p);
+    for (int k = 0; k < whole; ++k) used[p / 8 + k] = 8;
+    if (rest) used[p / 8 + whole] += rest;
+  }
+  if (fits) return;
+  at.clear();
+  int p = 0;
+  for (int b : order) {
+    at.push_back(p);
+    p += bs[b].width;
+  }
+}
+
 // One group planned by itself: its merge sets (group 0, slots and B image
 // counted from 0), to be placed into a launch by tc_append.
 struct TcGroupPlan {
@@ -288,6 +346,7 @@ inline int tc_plan_group(const TcGroupIn& g, int H, int S, TcGroupPlan& q) {
   if (S == 0) S = tc_choose_split(xs, g.D, g.max_split, H);
   if (S == 0) return -1;
   const int64_t Dp = (int64_t)S * g.D;
+  if (Dp > 65535) return -1;  // record field range
   q.g.D = (int)Dp;
   q.g.S = S;
   q.g.Wx = 0;
@@ -310,14 +369,19 @@ inline int tc_plan_group(const TcGroupIn& g, int H, int S, TcGroupPlan& q) {
     m.slot0 = (int16_t)q.slots.size();
     m.NS = (int16_t)NS;
     m.nchunks = (int16_t)nchunks;
-    m.R = (int16_t)(4 * NS <= 128 ? 2 : 1);
     int64_t Jmax = 0;
     bool range = true;
-    for (size_t b = i; b < j; ++b) {
-      const size_t n0 = q.slots.size();  // the bundle's first slot
-      tc_split_slots(xs, bs[b].first, bs[b].last, g.D, S, [&](const TcSlotX& x) {
+    std::vector<int> order, at;
+    tc_arrange(bs, i, j, NS, order, at);
+    q.slots.resize((size_t)m.slot0 + NS, TcSlot{});
+    q.slot_r.resize((size_t)m.slot0 + NS, 0);
+    for (size_t b = 0; b < order.size(); ++b) {
+      const TcBundle& bd = bs[order[b]];
+      const int n0 = at[b];  // the bundle's first position in the merge set
+      int n = n0;
+      tc_split_slots(xs, bd.first, bd.last, g.D, S, [&](const TcSlotX& x) {
         if (x.s.T > 65535 || x.s.U > 65535 || x.s.phi > 65535 || x.s.J > INT32_MAX) range = false;
-        TcSlot s{};
+        TcSlot& s = q.slots[(size_t)m.slot0 + n];
         s.w0 = (int32_t)x.start;
         s.J = (int32_t)x.s.J;
         s.ch = (uint16_t)x.s.ch;
@@ -325,19 +389,28 @@ inline int tc_plan_group(const TcGroupIn& g, int H, int S, TcGroupPlan& q) {
         s.U = (uint16_t)x.s.U;
         s.o = (uint16_t)(x.start + H - a);
         s.phi = (uint16_t)x.s.phi;
-        q.slots.push_back(s);
-        q.slot_r.push_back(x.s.r);
+        s.D = (uint16_t)Dp;
+        q.slot_r[(size_t)m.slot0 + n] = x.s.r;
         Jmax = std::max(Jmax, x.s.J);
+        ++n;
       });
-      // a slot at an even position followed by the channel's next output: one
-      // 16-byte store
-      for (size_t k = n0; k + 1 < q.slots.size(); ++k)
-        q.slots[k].flags = ((k - (size_t)m.slot0) % 2 == 0 && q.slot_r[k + 1] == q.slot_r[k] + 1) ? 1 : 0;
+      // how each position is stored: whole rows of 3, 5, 6 or 7 outputs in one
+      // chunk go through shared memory, else the widest aligned pieces
+      const TcSlot* sl = &q.slots[(size_t)m.slot0];
+      const int* r = &q.slot_r[(size_t)m.slot0];
+      const int W = sl[n0].U;
+      const bool run = n - n0 == W && W >= 3 && W <= 7 && W != 4 && n0 / 8 == (n - 1) / 8;
+      for (int k = n0; k < n; ++k) {
+        int f = 0;
+        if (k % 2 == 0 && k + 1 < n && r[k + 1] == r[k] + 1) f |= kTcPair;
+        if (k % 4 == 0 && k + 3 < n && W % 4 == 0 && r[k] % 4 == 0 && r[k + 3] == r[k] + 3) f |= kTcQuad;
+        if (run) f |= kTcRun | (W << 4) | ((k - n0) << 8);
+        q.slots[(size_t)m.slot0 + k].flags = (uint16_t)f;
+      }
     }
     if (!range) return -1;
-    q.slots.resize((size_t)m.slot0 + NS, TcSlot{});
-    q.slot_r.resize((size_t)m.slot0 + NS, 0);
     m.ntiles = (int32_t)((Jmax + kTcRows - 1) / kTcRows);
+    m.R = (int16_t)(4 * NS <= 128 ? 2 : 1);  // two narrow tiles an item share each B chunk
     m.items = (m.ntiles + m.R - 1) / m.R;
     m.b = q.b_bytes;
     q.b_bytes += (size_t)tc_round_up((int64_t)m.nchunks * 4 * NS * 128, 1024);
@@ -381,9 +454,15 @@ inline int tc_finish(TcPlan& p, int64_t N, int H, int num_sms) {
   if (sb > kTcStageMaxBytes) return -1;
   p.stage_bytes = sb;
   const int table = (int)tc_round_up((int64_t)p.slots.size() * kTcEpiSlotBytes, 1024);
-  p.stages = std::min(kTcMaxStages, (kTcSmemDyn - 1024 - table) / sb);
+  bool runs = false;
+  for (const TcSlot& x : p.slots) runs = runs || (x.flags & kTcRun) != 0;
+  p.scratch_warp = kTcEpiRecs + (runs ? kTcEpiRows : 0);  // (without runs: one more stage for narrow tiles)
+  const int scratch = kTcEpiWarps * p.scratch_warp;
+  p.stages = std::min(kTcMaxStages, (kTcSmemDyn - 1024 - table - scratch) / sb);
   if (p.stages < 2) return -1;
-  p.smem = p.stages * sb + table + 1024;
+  p.table_off = p.stages * sb;
+  p.scratch_off = p.table_off + table;
+  p.smem = p.scratch_off + scratch + 1024;
   // schedule: each CTA owns a contiguous range of input samples and runs the
   // items of every merge set that start in it, in input order
   int64_t umax = 0;
@@ -410,8 +489,8 @@ inline int tc_plan(const std::vector<TcGroupIn>& gin, int64_t N, int H, int num_
   return tc_finish(p, N, H, num_sms);
 }
 
-// Item range [first, last) of merge set m owned by CTA b (shared with the
-// device code: every role walks the same sequence).
+// Item range [first, last) of merge set m when each CTA owns an equal range of
+// input samples.
 FDSP_HD inline void tc_item_range(int64_t a, int64_t P, int64_t items, int64_t Lc, int b, int G, int64_t* first,
                           int64_t* last) {
   const int64_t v0 = (int64_t)b * Lc - a, v1 = (int64_t)(b + 1) * Lc - a;
@@ -419,6 +498,27 @@ FDSP_HD inline void tc_item_range(int64_t a, int64_t P, int64_t items, int64_t L
   int64_t l = v1 <= 0 ? 0 : (v1 + P - 1) / P;
   *first = f < items ? f : items;
   *last = (b == G - 1) ? items : (l < items ? l : items);
+}
+
+// Items of a merge set (first start a, step P) that start before sample lim:
+// summed over the merge sets, an item's place in the launch's item list.
+FDSP_HD inline uint32_t tc_items_before(uint32_t a, uint32_t P, uint32_t items, uint32_t lim) {
+  if (lim <= a) return 0;
+  const uint32_t n = (lim - a + P - 1u) / P;
+  return n < items ? n : items;
+}
+
+// Cost of an item in units of 32 cycles: 4 MMAs a chunk and tile, which took
+// 96 cycles at N = 128 and 168 at N = 256, and about 2000 cycles to start,
+// drain and store it.
+FDSP_HD inline uint32_t tc_item_cost(const TcMset& m) {
+  return ((uint32_t)m.R * (uint32_t)m.nchunks * (96u + 9u * (uint32_t)m.NS) + 2000u) / 32u;
+}
+
+// The items of CTA b of G are those whose cost before them lies in
+// [tc_cost_bound(b), tc_cost_bound(b + 1)).
+FDSP_HD inline uint32_t tc_cost_bound(uint32_t total, int b, int G) {
+  return (uint32_t)(((uint64_t)total * (uint64_t)b + (uint64_t)G - 1u) / (uint64_t)G);
 }
 
 }  // namespace fdsp
