@@ -104,34 +104,44 @@ int launch_cf32_to_ci16(const float2* in, int64_t n, short2* out, cudaStream_t s
 }
 
 // out[i - start] = atan2(Im, Re) of x[i] * conj(x[i-1]); x[-1] is the sample
-// saved by the previous apply (polar_discriminator.cc:150-165).
-__global__ void polar_kernel(const float2* __restrict__ in, int64_t N, const float2* __restrict__ prev, int start,
-                             float* __restrict__ out) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x + start;
-  if (i >= N) return;
-  const float2 a = in[i];
-  const float2 b = i > 0 ? in[i - 1] : *prev;
-  // a * conj(b), rounded like the reference's complex<float> product
-  const float re = a.x * b.x + a.y * b.y;
-  const float im = a.y * b.x - a.x * b.y;
-  out[i - start] = atan2f(im, re);
-}
+// saved by the previous apply (polar_discriminator.cc:150-165).  The last block
+// saves x[N-1] for the next one, into the other of two slots (another block
+// may still read this one's): a launch of its own took 2 us.  Bound by the
+// arc tangent's instructions: a thread's four outputs are independent chains.
+constexpr int kPolarThreads = 256;
+constexpr int kPolarPer = 4;
 
-__global__ void polar_save_kernel(const float2* __restrict__ in, int64_t N, float2* __restrict__ prev) {
-  *prev = in[N - 1];
-}
-
-int launch_polar(const float2* in, int64_t N, float2* d_prev, int start, float* out, cudaStream_t stream) {
-  if (N <= 0) return FDSP_OK;
-  const int64_t n_out = N - start;
-  if (n_out > 0) {
-    const int64_t nblocks = (n_out + 255) / 256;
-    if (nblocks > 0x7fffffffLL) return FDSP_ERR_UNSUPPORTED;
-    polar_kernel<<<(unsigned)nblocks, 256, 0, stream>>>(in, N, d_prev, start, out);
-    int st = cuda_status(cudaGetLastError());
-    if (st != FDSP_OK) return st;
+__global__ void __launch_bounds__(kPolarThreads)
+    polar_kernel(const float2* __restrict__ in, int64_t N, const float2* __restrict__ prev, float2* __restrict__ next,
+                 int start, float* __restrict__ out) {
+  const int64_t i0 = (int64_t)blockIdx.x * (kPolarThreads * kPolarPer) + threadIdx.x + start;
+  float2 a[kPolarPer], b[kPolarPer];
+#pragma unroll
+  for (int u = 0; u < kPolarPer; ++u) {
+    const int64_t i = i0 + u * kPolarThreads;
+    a[u] = b[u] = make_float2(0.f, 0.f);
+    if (i < N) {
+      a[u] = in[i];
+      b[u] = i > 0 ? in[i - 1] : *prev;
+    }
   }
-  polar_save_kernel<<<1, 1, 0, stream>>>(in, N, d_prev);
+#pragma unroll
+  for (int u = 0; u < kPolarPer; ++u) {
+    const int64_t i = i0 + u * kPolarThreads;
+    // a * conj(b), rounded like the reference's complex<float> product
+    const float re = a[u].x * b[u].x + a[u].y * b[u].y;
+    const float im = a[u].y * b[u].x - a[u].x * b[u].y;
+    if (i < N) out[i - start] = atan2f(im, re);
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *next = in[N - 1];
+}
+
+int launch_polar(const float2* in, int64_t N, const float2* d_prev, float2* d_next, int start, float* out,
+                 cudaStream_t stream) {
+  if (N <= 0) return FDSP_OK;
+  const int64_t per = kPolarThreads * kPolarPer, nblocks = std::max<int64_t>(1, (N - start + per - 1) / per);
+  if (nblocks > 0x7fffffffLL) return FDSP_ERR_UNSUPPORTED;
+  polar_kernel<<<(unsigned)nblocks, kPolarThreads, 0, stream>>>(in, N, d_prev, d_next, start, out);
   return cuda_status(cudaGetLastError());
 }
 
