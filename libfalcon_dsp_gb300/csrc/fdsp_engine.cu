@@ -258,12 +258,10 @@ __device__ __forceinline__ void win_finish(float2 acc, const ChanMeta& cm, const
 }
 
 template <bool kReal>
-__device__ __forceinline__ void process_rows_win(const float2* __restrict__ xs, const float4* __restrict__ tp,
-                                                 const ChanMeta* __restrict__ meta, int T, int D, int P, int a0,
-                                                 int jl0, int64_t j0, int64_t J, int U, int r, int delta) {
+__device__ __forceinline__ void win_sums(const float2* __restrict__ xs, const float4* __restrict__ tp, int T, int D,
+                                         int P, int a0, int jl0, f32x2 (&acc)[kWinRows]) {
   // packed multiply-adds in the scalar form's order: (re, re) (x, y), then
   // (-im, im) (y, x) for complex taps
-  f32x2 acc[kWinRows];
 #pragma unroll
   for (int q = 0; q < kWinRows; ++q) acc[q] = 0ull;
   const int bq = a0 / D, b0 = a0 - bq * D;
@@ -328,9 +326,6 @@ __device__ __forceinline__ void process_rows_win(const float2* __restrict__ xs, 
       }
     }
   }
-#pragma unroll
-  for (int q = 0; q < kWinRows; ++q)
-    if (j0 + q < J) win_finish(unpack2(acc[q]), meta[0], xs, tp, T, D, P, a0, jl0 + q, j0 + q, U, r, delta);
 }
 
 // History after a block: the last H samples of [old history | block], sample
@@ -504,6 +499,35 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
     // blocks fastest (Qt is a multiple of 32 kWinRows)
     const int nblk = Qt / kWinRows;
     const int nitems = nws * nblk;
+    f32x2 acc[kWinRows];
+    // One unshifted channel of one phase (FIR, integer decimation), a block a
+    // thread: the outputs go back through the tile's shared memory and leave
+    // in whole lines.  Stored from the registers, neighbouring lanes are 7
+    // outputs apart (a sector per 8 bytes), and each output paid a rotation:
+    // 64 complex taps over 2^20 samples, 26 us so, 18 us here.
+    if (nws == 1 && nblk <= kThreads && !meta_s[0].enabled && L.ws[G.ws_begin].U == 1) {
+      const WorkSet<NBMAX>& W = L.ws[G.ws_begin];
+      const int jl0 = (int)threadIdx.x * kWinRows;
+      const bool mine = (int)threadIdx.x < nblk && row0 + jl0 < W.J;
+      if (mine) {
+        const int a0 = (W.delta - G.delta_min) + (G.tmax - W.T);
+        const float4* tp = kTapsSmem ? taps_s + W.soff : W.taps;
+        if (G.real_taps)
+          win_sums<true>(xs, tp, W.T, D, P, a0, jl0, acc);
+        else
+          win_sums<false>(xs, tp, W.T, D, P, a0, jl0, acc);
+      }
+      float2* const out = meta_s[0].out;
+      __syncthreads();  // every window is summed: the tile is free
+      if (mine) {
+#pragma unroll
+        for (int q = 0; q < kWinRows; ++q) xs[jl0 + q] = cmul_nco(unpack2(acc[q]), make_float2(1.f, 0.f));
+      }
+      __syncthreads();
+      const int rows = (int)min((int64_t)Qt, W.J - row0);
+      for (int i = threadIdx.x; i < rows; i += kThreads) out[row0 + i] = xs[i];
+      return;
+    }
     for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
       const int wq = it / nblk;
       const int jl0 = (it - wq * nblk) * kWinRows;
@@ -515,9 +539,13 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
       const float4* tp = kTapsSmem ? taps_s + W.soff : W.taps;
       const ChanMeta* mt = meta_s + wq * NBMAX;
       if (G.real_taps)
-        process_rows_win<true>(xs, tp, mt, T, D, P, a0, jl0, j0, W.J, W.U, W.r, W.delta);
+        win_sums<true>(xs, tp, T, D, P, a0, jl0, acc);
       else
-        process_rows_win<false>(xs, tp, mt, T, D, P, a0, jl0, j0, W.J, W.U, W.r, W.delta);
+        win_sums<false>(xs, tp, T, D, P, a0, jl0, acc);
+#pragma unroll
+      for (int q = 0; q < kWinRows; ++q)
+        if (j0 + q < W.J)
+          win_finish(unpack2(acc[q]), mt[0], xs, tp, T, D, P, a0, jl0 + q, j0 + q, W.U, W.r, W.delta);
     }
     return;
   }
