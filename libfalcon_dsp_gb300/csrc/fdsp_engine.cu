@@ -362,6 +362,7 @@ template <int NBMAX, bool kTapsSmem, bool kWin>
 __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
     poly_fp32_kernel(const __grid_constant__ PolyLaunch<NBMAX> L, int first, int tiles) {
   extern __shared__ __align__(16) float2 xs[];
+  grid_dependency();
   int tile = blockIdx.x;
   if (tile >= tiles) {
     const int i = (tile - tiles) * kThreads + (int)threadIdx.x;
@@ -604,6 +605,7 @@ constexpr int kNatMaxCols = 512;   // threads of a CTA: a multiple of U columns,
 template <bool kCheck>
 __global__ void __launch_bounds__(kNatMaxCols) nat_resample_kernel(const __grid_constant__ NatLaunch L, int tiles) {
   extern __shared__ __align__(16) float2 xs[];
+  grid_dependency();
   const int threads = (int)blockDim.x;
   if ((int)blockIdx.x >= tiles) {
     const int i = ((int)blockIdx.x - tiles) * threads + (int)threadIdx.x;
@@ -706,6 +708,23 @@ __global__ void hist_update_kernel(const float2* __restrict__ old_hist, const fl
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+cudaError_t launch_overlapped(const void* func, dim3 grid, dim3 block, size_t smem, cudaStream_t s, void** args) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  const bool known = cudaStreamIsCapturing(s, &cs) == cudaSuccess;
+  if (!known) cudaGetLastError();
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = known && cs == cudaStreamCaptureStatusNone ? 1u : 0u;
+  return cudaLaunchKernelExC(&cfg, func, args);
+}
+
 NcoConst make_nco(uint32_t fs, int32_t f) {
   NcoConst n;
   std::memset(&n, 0, sizeof(n));
@@ -1479,7 +1498,7 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
       hist_blocks = (H_ + kThreads - 1) / kThreads;
       hist_done = true;
     }
-    e = klaunch(bt.kern, dim3((unsigned)(tiles + hist_blocks)), dim3(kThreads), bt.smem, stream, L, first, tiles);
+    e = klaunch_overlapped(bt.kern, dim3((unsigned)(tiles + hist_blocks)), dim3(kThreads), bt.smem, stream, L, first, tiles);
     if (kprof_) cudaEventRecord(kprof_event(), stream);
     if (e != cudaSuccess) return cuda_status(e);
     launches_last_++;
@@ -1545,7 +1564,7 @@ int PolyEngine::launch_nat(const float2* d_in, uint64_t n, float2* out, bool che
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_status(e);
   if (kprof_) cudaEventRecord(kprof_event(), stream);
-  e = klaunch(kern, dim3((unsigned)(tiles + hist_blocks)), dim3((unsigned)threads), smem, stream, L, tiles);
+  e = klaunch_overlapped(kern, dim3((unsigned)(tiles + hist_blocks)), dim3((unsigned)threads), smem, stream, L, tiles);
   if (kprof_) cudaEventRecord(kprof_event(), stream);
   if (e != cudaSuccess) return cuda_status(e);
   launches_last_++;

@@ -68,6 +68,7 @@ __device__ __forceinline__ float deemph_step(float x, float y, float b0, float c
 __global__ void __launch_bounds__(kFmThreads) fm_polar_deemph_kernel(const FmLaunch L) {
   __shared__ float pol[kFmWarm + kFmTile + (kFmWarm + kFmTile) / kFmPer];
   __shared__ float res[kFmTile + kFmTile / kFmPer];
+  grid_dependency();
   const int64_t t0 = (int64_t)blockIdx.x * kFmTile;
   const int64_t h0 = t0 - kFmWarm;  // discriminator output held in pol[0]
   for (int i = threadIdx.x; i < kFmWarm + kFmTile; i += kFmThreads) {
@@ -136,6 +137,7 @@ constexpr int64_t kFmOneMax = 1 << 17;
 __global__ void __cluster_dims__(kFmCluster, 1, 1) __launch_bounds__(512)
     fm_normalize_kernel(const float2* m, int64_t n, int16_t* out) {
   __shared__ unsigned smax;
+  grid_dependency();
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   if (threadIdx.x == 0) smax = 0u;
@@ -303,8 +305,9 @@ int fdsp_fm_demod_apply(fdsp_fm_demod* h, const fdsp_cf32* d_in, uint64_t n_in, 
     L.c = h->c;
     L.out = iir;
     const int64_t blocks = std::max<int64_t>(1, ((int64_t)c.pol + kFmTile - 1) / kFmTile);
-    fm_polar_deemph_kernel<<<(unsigned)blocks, kFmThreads, 0, s>>>(L);
-    FDSP_TRY(cuda_status(cudaGetLastError()));
+    void* args[] = {&L};
+    FDSP_TRY(cuda_status(launch_overlapped(reinterpret_cast<const void*>(fm_polar_deemph_kernel),
+                                           dim3((unsigned)blocks), dim3(kFmThreads), 0, s, args)));
     h->cur ^= 1;
     h->have_prev = true;
   }
@@ -312,8 +315,11 @@ int fdsp_fm_demod_apply(fdsp_fm_demod* h, const fdsp_cf32* d_in, uint64_t n_in, 
   FDSP_TRY(fdsp_resampler_apply(h->mono, reinterpret_cast<const fdsp_cf32*>(iir), c.pol,
                                 reinterpret_cast<fdsp_cf32*>(mono), c.mono + 1, &nm, stream));
   if (c.mono > 0 && c.mono <= (uint64_t)kFmOneMax) {
-    fm_normalize_kernel<<<kFmCluster, 512, 0, s>>>(mono, (int64_t)c.mono, d_out);
-    FDSP_TRY(cuda_status(cudaGetLastError()));
+    const float2* a0 = mono;
+    int64_t a1 = (int64_t)c.mono;
+    void* args[] = {&a0, &a1, &d_out};
+    FDSP_TRY(cuda_status(launch_overlapped(reinterpret_cast<const void*>(fm_normalize_kernel), dim3(kFmCluster),
+                                           dim3(512), 0, s, args)));
   } else if (c.mono > 0) {
     unsigned* amax = reinterpret_cast<unsigned*>(h->d_state + 4);
     FDSP_TRY(cuda_status(cudaMemsetAsync(amax, 0, sizeof(unsigned), s)));

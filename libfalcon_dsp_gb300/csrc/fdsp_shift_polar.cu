@@ -32,6 +32,7 @@ constexpr int kShiftTile = kShiftThreads * kShiftPer;
 
 __global__ void __launch_bounds__(kShiftThreads)
     freq_shift_kernel(const __grid_constant__ ShiftLaunch L) {
+  grid_dependency();
   const int64_t t0 = (int64_t)blockIdx.x * kShiftTile;
   float2 x[kShiftPer];
 #pragma unroll
@@ -85,8 +86,9 @@ int launch_freq_shift(const ShiftLaunch& L, cudaStream_t stream) {
   if (L.N <= 0) return FDSP_OK;
   const int64_t nblocks = (L.N + kShiftTile - 1) / kShiftTile;
   if (nblocks > 0x7fffffffLL) return FDSP_ERR_UNSUPPORTED;
-  freq_shift_kernel<<<(unsigned)nblocks, kShiftThreads, 0, stream>>>(L);
-  return cuda_status(cudaGetLastError());
+  void* args[] = {const_cast<ShiftLaunch*>(&L)};
+  return cuda_status(launch_overlapped(reinterpret_cast<const void*>(freq_shift_kernel), dim3((unsigned)nblocks),
+                                       dim3(kShiftThreads), 0, stream, args));
 }
 
 __global__ void cf32_to_ci16_kernel(const float2* __restrict__ in, int64_t n, short2* __restrict__ out) {
@@ -114,6 +116,7 @@ constexpr int kPolarPer = 4;
 __global__ void __launch_bounds__(kPolarThreads)
     polar_kernel(const float2* __restrict__ in, int64_t N, const float2* __restrict__ prev, float2* __restrict__ next,
                  int start, float* __restrict__ out) {
+  grid_dependency();
   const int64_t i0 = (int64_t)blockIdx.x * (kPolarThreads * kPolarPer) + threadIdx.x + start;
   float2 a[kPolarPer], b[kPolarPer];
 #pragma unroll
@@ -141,8 +144,9 @@ int launch_polar(const float2* in, int64_t N, const float2* d_prev, float2* d_ne
   if (N <= 0) return FDSP_OK;
   const int64_t per = kPolarThreads * kPolarPer, nblocks = std::max<int64_t>(1, (N - start + per - 1) / per);
   if (nblocks > 0x7fffffffLL) return FDSP_ERR_UNSUPPORTED;
-  polar_kernel<<<(unsigned)nblocks, kPolarThreads, 0, stream>>>(in, N, d_prev, d_next, start, out);
-  return cuda_status(cudaGetLastError());
+  void* args[] = {&in, &N, &d_prev, &d_next, &start, &out};
+  return cuda_status(launch_overlapped(reinterpret_cast<const void*>(polar_kernel), dim3((unsigned)nblocks),
+                                       dim3(kPolarThreads), 0, stream, args));
 }
 
 }  // namespace fdsp
