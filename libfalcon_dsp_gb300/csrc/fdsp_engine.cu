@@ -104,7 +104,7 @@ __device__ __forceinline__ void process_rows(const float2* __restrict__ xs, cons
     for (int n = 0; n < NB; ++n) sa[q][n] = sb[q][n] = 0ull;
   // runs of taps between the wraps of the de-interleaved tile
   for (int k = 0, end = min(T, nph - b0); k < T; end = min(T, k + nph), xp += wrap) {
-#pragma unroll 2
+#pragma unroll(NB > 4 ? 1 : 2)
     for (; k < end; ++k) {
       f32x2 x[kRows];
 #pragma unroll
@@ -218,8 +218,9 @@ __device__ __forceinline__ void process_block(int rows, const float2* __restrict
 // semantics) take 2 FMAs per tap instead of 4.
 constexpr int kWinRows = 7;
 
-// Shared memory of a CTA that leaves room for two more on the SM.
+// Shared memory of a CTA that leaves room for two more, or one more, on the SM.
 constexpr int kSmem3 = 75 * 1024;
+constexpr int kSmem2 = 112 * 1024;
 
 // Rotation and store of one single-channel output (the per-row epilogue
 // for NB = 1).
@@ -297,12 +298,26 @@ __device__ __forceinline__ void win_sums(const float2* __restrict__ xs, const fl
     for (int q = 0; q < kWinRows - 1; ++q) put(q, xr[q]);
     int m = 0;
     for (; m + kWinRows <= nm; m += kWinRows) {
-      // circular window: sample m + u + q sits in slot (u + q) % kWinRows
+      // circular window: sample m + u + q sits in slot (u + q) % kWinRows; real
+      // taps leave the registers to read the block's taps and samples first
+      f32x2 xn[kReal ? kWinRows : 1], gn[kReal ? kWinRows : 1];
+      if constexpr (kReal) {
+#pragma unroll
+        for (int u = 0; u < kWinRows; ++u) {
+          xn[u] = xr[m + u + kWinRows - 1];
+          gn[u] = tk[(m + u) * D].x;
+        }
+      }
 #pragma unroll
       for (int u = 0; u < kWinRows; ++u) {
-        put((u + kWinRows - 1) % kWinRows, xr[m + u + kWinRows - 1]);
         f32x2 gr, gi = 0ull;
-        tap(m + u, gr, gi);
+        if constexpr (kReal) {
+          put((u + kWinRows - 1) % kWinRows, xn[u]);
+          gr = gn[u];
+        } else {
+          put((u + kWinRows - 1) % kWinRows, xr[m + u + kWinRows - 1]);
+          tap(m + u, gr, gi);
+        }
 #pragma unroll
         for (int q = 0; q < kWinRows; ++q) {
           acc[q] = fma2(gr, w[(u + q) % kWinRows], acc[q]);
@@ -876,10 +891,16 @@ int PolyEngine::init(uint32_t fs, const fdsp_channel_cfg* ch, uint32_t nch, bool
   }
   H_ = tmax_all - 1;
 
-  // NB: channels per tap batch (largest class decides, power of two <= 8)
-  size_t maxcls = 1;
-  for (auto& k : classes_) maxcls = std::max(maxcls, k.chans.size());
-  nb_ = maxcls >= 8 ? 8 : maxcls >= 4 ? 4 : maxcls >= 2 ? 2 : 1;
+  // NB: channels per tap batch (largest class decides).  Four: the kernel then
+  // keeps three CTAs an SM (eight leave two: 256 channels of 2^26 samples took
+  // 18.9 ms by eight and 15.9 by four); eight only where batches of four would
+  // exceed a launch's work sets.
+  size_t maxcls = 1, sets4 = 0;
+  for (auto& k : classes_) {
+    maxcls = std::max(maxcls, k.chans.size());
+    sets4 += (k.chans.size() + 3) / 4 * k.up;
+  }
+  nb_ = maxcls >= 8 && sets4 > (size_t)kMaxWorkSets ? 8 : maxcls >= 4 ? 4 : maxcls >= 2 ? 2 : 1;
 
   // decimation groups
   std::map<uint32_t, int> gidx;
@@ -1391,23 +1412,26 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
     ng++;
   }
   // Blocks too short to give every SM three tiles of the default height take
-  // lower tiles (latency: more of the GPU stages and computes at once).
+  // lower tiles (latency: more of the GPU stages and computes at once), but not
+  // so low that a tile stages more halo than rows (4095 taps by 10 over 2^20
+  // samples: 0.93 ms with 32 rows, 0.34 with 384).
   for (int shift = 1; shift <= 5; ++shift) {
     int64_t tiles = 0;
     for (int gi = 0; gi < ng; ++gi) tiles += (rows_of[gi] + qt_of[gi] - 1) / qt_of[gi];
     if (tiles >= 3LL * num_sms_) break;
     for (int gi = 0; gi < ng; ++gi)
-      if (!fixed_qt[gi]) qt_of[gi] = std::max(32, (qt_of[gi] / 2) & ~31);
+      if (!fixed_qt[gi] &&
+          (int64_t)(qt_of[gi] / 2) * L.groups[gi].D >= (int64_t)L.groups[gi].tmax + L.groups[gi].delta_span)
+        qt_of[gi] = std::max(32, (qt_of[gi] / 2) & ~31);
   }
   for (int gi = 0; gi < ng; ++gi) {
     GroupDesc& gd = L.groups[gi];
-    for (;;) {  // a lower tile where this one leaves no room for two more CTAs (or is over the limit)
+    for (;;) {  // a lower tile where this one's samples leave no room for the other CTAs (or it is over the limit)
       layout_group<NB>(L, gd, qt_of[gi]);
-      if (gd.smem_bytes <= (fixed_qt[gi] ? 227 * 1024 : kSmem3)) break;
-      if (gd.win || qt_of[gi] <= 32) {
-        if (gd.smem_bytes > 227 * 1024) return FDSP_ERR_UNSUPPORTED;
-        break;
-      }
+      const int roomy = NB == 8 ? kSmem2 : kSmem3;  // (registers allow two CTAs of 8-channel batches, three of others)
+      const bool trim = !fixed_qt[gi] && gd.smem_bytes > roomy && 16 * (int64_t)gd.taps_off > gd.smem_bytes;
+      if (gd.smem_bytes <= 227 * 1024 && (!trim || qt_of[gi] <= 32)) break;
+      if (gd.win || qt_of[gi] <= 32) return FDSP_ERR_UNSUPPORTED;
       qt_of[gi] -= 32;
     }
     gd.ntiles = (int32_t)((rows_of[gi] + gd.Qt - 1) / gd.Qt);
@@ -1457,12 +1481,14 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
     }
     std::sort(order, order + nfp, [&](int a, int b) { return cost[a] != cost[b] ? cost[a] > cost[b] : a < b; });
     const bool single = !prof_ev_.empty() || (done_fn_ && tiles > 3LL * num_sms_);
-    for (int variant = 0; variant < 8; ++variant) {
-      const bool smem_taps = (variant & 1) == 0, win = (variant & 2) != 0, big = (variant & 4) != 0;
+    for (int variant = 0; variant < 12; ++variant) {
+      const bool smem_taps = (variant & 1) == 0, win = (variant & 2) != 0;
+      const int size = variant >> 2;  // CTAs that fit an SM: three or more, two, one
       bool open = false;
       for (int i = 0; i < nfp; ++i) {
         const GroupDesc& gd = L.groups[order[i]];
-        if ((gd.taps_smem != 0) != smem_taps || (gd.win != 0) != win || (gd.smem_bytes > kSmem3) != big) continue;
+        if ((gd.taps_smem != 0) != smem_taps || (gd.win != 0) != win || (gd.smem_bytes > kSmem3) + (gd.smem_bytes > kSmem2) != size)
+          continue;
         if (!open || single) {
           Batch& nb = lb[nlb++];
           nb.kern = win ? (smem_taps ? reinterpret_cast<const void*>(poly_fp32_kernel<NB, true, true>)
