@@ -516,15 +516,16 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
     const int nblk = Qt / kWinRows;
     const int nitems = nws * nblk;
     f32x2 acc[kWinRows];
-    // One unshifted channel of one phase (FIR, integer decimation), a block a
-    // thread: the outputs go back through the tile's shared memory and leave
-    // in whole lines.  Stored from the registers, neighbouring lanes are 7
-    // outputs apart (a sector per 8 bytes), and each output paid a rotation:
+    // One unshifted channel, a block a thread: the tile's outputs (every phase
+    // of every row, contiguous in the channel) go back through shared memory
+    // and leave in whole lines.  Stored from the registers, neighbouring lanes
+    // are 7 rows apart (a sector per 8 bytes), and each output paid a rotation:
     // 64 complex taps over 2^20 samples, 26 us so, 18 us here.
-    if (nws == 1 && nblk <= kThreads && !meta_s[0].enabled && L.ws[G.ws_begin].U == 1) {
-      const WorkSet<NBMAX>& W = L.ws[G.ws_begin];
-      const int jl0 = (int)threadIdx.x * kWinRows;
-      const bool mine = (int)threadIdx.x < nblk && row0 + jl0 < W.J;
+    if (G.lines) {
+      const int wq = (int)threadIdx.x / nblk, U = nws;
+      const int jl0 = ((int)threadIdx.x - wq * nblk) * kWinRows;
+      const WorkSet<NBMAX>& W = L.ws[G.ws_begin + min(wq, nws - 1)];
+      const bool mine = wq < nws && row0 + jl0 < W.J;
       if (mine) {
         const int a0 = (W.delta - G.delta_min) + (G.tmax - W.T);
         const float4* tp = kTapsSmem ? taps_s + W.soff : W.taps;
@@ -533,15 +534,16 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
         else
           win_sums<false>(xs, tp, W.T, D, P, a0, jl0, acc);
       }
-      float2* const out = meta_s[0].out;
+      float2* const out = meta_s[0].out + row0 * U;
       __syncthreads();  // every window is summed: the tile is free
       if (mine) {
 #pragma unroll
-        for (int q = 0; q < kWinRows; ++q) xs[jl0 + q] = cmul_nco(unpack2(acc[q]), make_float2(1.f, 0.f));
+        for (int q = 0; q < kWinRows; ++q)
+          xs[(jl0 + q) * U + W.r] = cmul_nco(unpack2(acc[q]), make_float2(1.f, 0.f));
       }
       __syncthreads();
-      const int rows = (int)min((int64_t)Qt, W.J - row0);
-      for (int i = threadIdx.x; i < rows; i += kThreads) out[row0 + i] = xs[i];
+      const int count = (int)min((int64_t)Qt * U, G.outs - row0 * U);
+      for (int i = threadIdx.x; i < count; i += kThreads) out[i] = xs[i];
       return;
     }
     for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
@@ -1319,6 +1321,7 @@ static void layout_group(PolyLaunch<NB>& L, GroupDesc& gd, int Qt) {
   gd.P = (int32_t)P;
   // shared-memory layout: input tile | taps of each work set | channel constants
   int64_t off = ((int64_t)gd.nph * P + 1) & ~1LL;  // float2 units, 16-byte aligned
+  if (gd.lines) off = std::max(off, (int64_t)Qt * (gd.ws_end - gd.ws_begin));  // the tile's outputs take its place
   gd.taps_off = (int32_t)off;
   int64_t toff = 0;
   for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) {
@@ -1402,8 +1405,16 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
     const bool win = g.win && rows >= (int64_t)g.Qt_win * num_sms_;
     gd.win = win ? 1 : 0;
     gd.real_taps = g.real_taps;
+    // one unshifted channel whose every phase has outputs, a block of rows a
+    // thread, the outputs within the tile's budget
+    const int nsets = nws - gd.ws_begin, unit = 32 * kWinRows;
+    const int qt_lines = std::min(g.Qt_win, std::max(1, kThreads / nsets) * kWinRows / unit * unit);
+    gd.lines = win && g.batches.size() == 1 && !chans_[batches_[g.batches[0]].chans[0]].nco.enabled &&
+               nsets == (int)classes_[batches_[g.batches[0]].cls].up && qt_lines >= unit &&
+               (int64_t)nsets * qt_lines * 8 <= 64 * 1024;
+    gd.outs = gd.lines ? (int64_t)classes_[batches_[g.batches[0]].cls].M : 0;
     rows_of[ng] = rows;
-    qt_of[ng] = win ? g.Qt_win : g.Qt;
+    qt_of[ng] = gd.lines ? qt_lines : win ? g.Qt_win : g.Qt;
     if (!win && g.Qt == g.Qt_default && g.Qt == 32) {  // two rows a thread where the windows' phases alone fit
       layout_group<NB>(L, gd, 64);
       if (gd.smem_bytes <= kSmem3) qt_of[ng] = 64;

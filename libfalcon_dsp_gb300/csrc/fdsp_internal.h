@@ -73,6 +73,8 @@ struct GroupDesc {
   int32_t seg_at[kMaxSegs - 1];   // staged phase where a gap lies (INT32_MAX: none)
   int32_t seg_gap[kMaxSegs - 1];  // unstaged phases of that gap
   int32_t step_q, step_b;  // kThreads staged samples on: rows and phases
+  int32_t lines;      // sliding window: outputs leave through shared memory
+  int64_t outs;       // outputs of the channel (lines)
   int32_t span;       // input samples from the first staged one to past the last
   uint64_t inv_nph;   // ceil(2^32 / nph): t / nph as one multiply and shift
 };

@@ -43,6 +43,19 @@ def test_decimator(down, taps):
         assert y.size == r.size and rel_rms(y, r) <= 1e-5
 
 
+@pytest.mark.parametrize("up,down,tpp", [(3, 2, 60), (2, 5, 17), (7, 8, 33), (5, 3, 16)])
+def test_rational(up, down, tpp):
+    """The few-phase rates: every phase of a tile's rows leaves together."""
+    import torch
+    rng = np.random.default_rng(up * 10 + down)
+    h = (rng.standard_normal(up * tpp) / np.sqrt(tpp)).astype(np.complex64)
+    f, o = F.PolyphaseResamplerCuda(up, down, h), O.Resampler(up, down, h)
+    for n in (TILE * 160 * down + 1, TILE * 155 * down - 1, TILE * 170 * down + 2):
+        x = _x(rng, n)
+        y, r = f.apply(torch.from_numpy(x).cuda()).cpu().numpy(), o.apply(x)
+        assert y.size == r.size and rel_rms(y, r) <= 1e-5
+
+
 def test_infinite_sample_marks_its_window():
     import torch
     n, taps = TILE * 160, 64
