@@ -158,11 +158,6 @@ struct TcRing {
   }
 };
 
-// Input samples between the starts of a merge set's items.
-__device__ __forceinline__ uint32_t tc_item_step(const TcMset& M, const TcGroup* groups) {
-  return (uint32_t)M.R * (uint32_t)kTcRows * (uint32_t)groups[M.group].D;
-}
-
 // ---------------------------------------------------------------------------
 // prep: split [history | block] into {hi, lo} parts, build the B images and
 // the item list
@@ -217,9 +212,8 @@ __global__ void __launch_bounds__(256) tc_prep_kernel(const __grid_constant__ Tc
       uint8_t* dst = L.bbuf + M.b + ((size_t)c * N + n) * 128 + (size_t)((q ^ (n & 7)) * 16);
       *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    // the items in the order of their first input sample (ties: the lower
-    // merge set), each with the cost of all items before it: a division per
-    // merge set gives both
+    // the items in the order of their first input sample, each with the cost
+    // of all items before it
     const int nitems = L.iprefix[L.nmsets];
     for (int p = (int)blockIdx.x * 256 + (int)threadIdx.x; p < nitems; p += nb_build * 256) {
       int m = 0, hi = L.nmsets;  // largest m with iprefix[m] <= p
@@ -229,15 +223,8 @@ __global__ void __launch_bounds__(256) tc_prep_kernel(const __grid_constant__ Tc
         else hi = mid;
       }
       const int t = p - L.iprefix[m];
-      const uint32_t u = (uint32_t)L.ms[m].a + (uint32_t)t * tc_item_step(L.ms[m], L.groups);
-      uint32_t place = 0, cost = 0;
-      for (int k = 0; k < L.nmsets; ++k) {
-        // (items of k that start before this one; at the same sample the lower merge set goes first)
-        const uint32_t before = tc_items_before((uint32_t)L.ms[k].a, tc_item_step(L.ms[k], L.groups),
-                                                (uint32_t)L.ms[k].items, u + (k < m ? 1u : 0u));
-        place += before;
-        cost += before * tc_item_cost(L.ms[k]);
-      }
+      uint32_t place, cost;
+      tc_item_place(L.ms, L.nmsets, L.groups, m, t, L.cost_shift, &place, &cost);
       L.items[place] = make_uint2(((uint32_t)m << 26) | (uint32_t)t, cost);
     }
     return;
@@ -1200,7 +1187,8 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
       items += plan.ms[m].items;
     }
     L.iprefix[plan.ms.size()] = items;
-    for (const TcMset& m : plan.ms) L.ctotal += (uint32_t)m.items * tc_item_cost(m);
+    L.ctotal = plan.ctotal;
+    L.cost_shift = plan.cost_shift;
     for (size_t s = 0; s < plan.slots.size(); ++s) {
       L.slots[s] = plan.slots[s];
       if (plan.slots[s].J > 0)

@@ -160,9 +160,10 @@ struct TcLaunch {
   int32_t bprefix[kTcMaxMsets + 1];  // 16-byte pieces of the B images before merge set m
   int32_t iprefix[kTcMaxMsets + 1];  // items before merge set m
   uint2* items;                      // every item by first input sample: {merge set << 26 | item, cost before it} (prep writes it)
-  uint32_t ctotal;                   // cost of all items
+  uint32_t ctotal;                   // cost of all items, below 2^31
+  int32_t cost_shift;                // its unit (TcPlan::cost_shift)
   int32_t scratch_warp;              // scratch bytes of an epilogue warp: rows of runs (if any), then records
-  uint32_t pad_[2];
+  uint32_t pad_;
   TcGroup groups[kTcMaxGroups];
   TcMset ms[kTcMaxMsets];
   TcSlot slots[kTcMaxSlots];

@@ -130,6 +130,8 @@ struct TcPlan {
   int G = 0;                      // grid (CTAs)
   int64_t Lc = 0;                 // samples of the time range each CTA owns
   int64_t items = 0;
+  uint32_t ctotal = 0;            // cost of all items, each at least 1 and scaled by 2^-cost_shift
+  int cost_shift = 0;
 };
 
 inline int64_t tc_round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
@@ -438,6 +440,51 @@ inline bool tc_append(TcPlan& p, const TcGroupPlan& q) {
   return true;
 }
 
+// Items of a merge set (first start a, step P) that start before sample lim:
+// summed over the merge sets, an item's place in the launch's item list.
+FDSP_HD inline uint32_t tc_items_before(uint32_t a, uint32_t P, uint32_t items, uint32_t lim) {
+  if (lim <= a) return 0;
+  const uint32_t n = (lim - a + P - 1u) / P;
+  return n < items ? n : items;
+}
+
+// Cost of an item in units of 32 cycles: 4 MMAs a chunk and tile, which took
+// 96 cycles at N = 128 and 168 at N = 256, and about 2000 cycles to start,
+// drain and store it; in units of 2^shift as much for launches of more work.
+// Never 0, so costs grow along the item list.
+FDSP_HD inline uint32_t tc_item_cost(const TcMset& m, int shift = 0) {
+  const uint32_t c = (((uint32_t)m.R * (uint32_t)m.nchunks * (96u + 9u * (uint32_t)m.NS) + 2000u) / 32u) >> shift;
+  return c > 0u ? c : 1u;
+}
+
+// Input samples between the starts of a merge set's items.
+template <class Group>
+FDSP_HD inline uint32_t tc_item_step(const TcMset& m, const Group* groups) {
+  return (uint32_t)m.R * (uint32_t)kTcRows * (uint32_t)groups[m.group].D;
+}
+
+// Where item t of merge set m stands in the list of all items, ordered by
+// first input sample (ties: the lower merge set), and the cost of the items
+// before it: a division per merge set gives both.
+template <class Group>
+FDSP_HD inline void tc_item_place(const TcMset* ms, int nmsets, const Group* groups, int m, int t, int shift,
+                                  uint32_t* place, uint32_t* cost) {
+  const uint32_t u = (uint32_t)ms[m].a + (uint32_t)t * tc_item_step(ms[m], groups);
+  *place = *cost = 0;
+  for (int k = 0; k < nmsets; ++k) {
+    const uint32_t before =
+        tc_items_before((uint32_t)ms[k].a, tc_item_step(ms[k], groups), (uint32_t)ms[k].items, u + (k < m ? 1u : 0u));
+    *place += before;
+    *cost += before * tc_item_cost(ms[k], shift);
+  }
+}
+
+// The items of CTA b of G are those whose cost before them lies in
+// [tc_cost_bound(b), tc_cost_bound(b + 1)).
+FDSP_HD inline uint32_t tc_cost_bound(uint32_t total, int b, int G) {
+  return (uint32_t)(((uint64_t)total * (uint64_t)b + (uint64_t)G - 1u) / (uint64_t)G);
+}
+
 // Sizes and schedule of a launch whose groups are all added.  Returns 0, or
 // -1 when its stages do not fit shared memory.
 inline int tc_finish(TcPlan& p, int64_t N, int H, int num_sms) {
@@ -473,6 +520,17 @@ inline int tc_finish(TcPlan& p, int64_t N, int H, int num_sms) {
   }
   p.G = (int)std::max<int64_t>(1, std::min<int64_t>(num_sms, p.items));
   p.Lc = (umax + p.G - 1) / p.G;
+  // The CTAs' cuts and the costs in the item list are 32-bit: the unit of cost
+  // doubles until the total stays below 2^31 (only calls of half a second of
+  // work and more, such as 4095 taps of 32 channels over 2^31 samples, need it).
+  uint64_t total = 0;
+  for (p.cost_shift = 0;; ++p.cost_shift) {
+    total = 0;
+    for (const TcMset& m : p.ms) total += (uint64_t)m.items * tc_item_cost(m, p.cost_shift);
+    if (total < (1ull << 31) || p.cost_shift == 31) break;
+  }
+  if (total >= (1ull << 31)) return -1;
+  p.ctotal = (uint32_t)total;
   return 0;
 }
 
@@ -498,27 +556,6 @@ FDSP_HD inline void tc_item_range(int64_t a, int64_t P, int64_t items, int64_t L
   int64_t l = v1 <= 0 ? 0 : (v1 + P - 1) / P;
   *first = f < items ? f : items;
   *last = (b == G - 1) ? items : (l < items ? l : items);
-}
-
-// Items of a merge set (first start a, step P) that start before sample lim:
-// summed over the merge sets, an item's place in the launch's item list.
-FDSP_HD inline uint32_t tc_items_before(uint32_t a, uint32_t P, uint32_t items, uint32_t lim) {
-  if (lim <= a) return 0;
-  const uint32_t n = (lim - a + P - 1u) / P;
-  return n < items ? n : items;
-}
-
-// Cost of an item in units of 32 cycles: 4 MMAs a chunk and tile, which took
-// 96 cycles at N = 128 and 168 at N = 256, and about 2000 cycles to start,
-// drain and store it.
-FDSP_HD inline uint32_t tc_item_cost(const TcMset& m) {
-  return ((uint32_t)m.R * (uint32_t)m.nchunks * (96u + 9u * (uint32_t)m.NS) + 2000u) / 32u;
-}
-
-// The items of CTA b of G are those whose cost before them lies in
-// [tc_cost_bound(b), tc_cost_bound(b + 1)).
-FDSP_HD inline uint32_t tc_cost_bound(uint32_t total, int b, int G) {
-  return (uint32_t)(((uint64_t)total * (uint64_t)b + (uint64_t)G - 1u) / (uint64_t)G);
 }
 
 }  // namespace fdsp
