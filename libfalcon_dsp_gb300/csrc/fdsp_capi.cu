@@ -138,8 +138,7 @@ struct fdsp_freq_shift {
 };
 
 struct fdsp_polar {
-  float2* d_prev = nullptr;  // two slots in turn: a call reads x[-1] from one and saves its last sample in the other
-  int cur = 0;
+  float2* d_prev = nullptr;  // x[-1]
   bool have_prev = false;
   DevBuf in, out;
   ~fdsp_polar() {
@@ -802,8 +801,8 @@ int fdsp_polar_create(fdsp_polar** out) {
   *out = nullptr;
   fdsp_polar* h = new (std::nothrow) fdsp_polar();
   if (!h) return FDSP_ERR_ALLOC;
-  cudaError_t e = cudaMalloc(&h->d_prev, 2 * sizeof(float2));
-  if (e == cudaSuccess) e = cudaMemset(h->d_prev, 0, 2 * sizeof(float2));
+  cudaError_t e = cudaMalloc(&h->d_prev, sizeof(float2));
+  if (e == cudaSuccess) e = cudaMemset(h->d_prev, 0, sizeof(float2));
   if (e != cudaSuccess) {
     delete h;
     return cuda_status(e);
@@ -839,9 +838,8 @@ int fdsp_polar_apply(fdsp_polar* h, const fdsp_cf32* d_in, uint64_t n_in, float*
   if (n_out) *n_out = cnt;
   if (n_in == 0) return FDSP_OK;
   if (!d_in || (cnt > 0 && !d_out)) return FDSP_ERR_INVALID_ARG;
-  FDSP_TRY(launch_polar(reinterpret_cast<const float2*>(d_in), (int64_t)n_in, h->d_prev + h->cur,
-                        h->d_prev + (h->cur ^ 1), h->have_prev ? 0 : 1, d_out, (cudaStream_t)stream));
-  h->cur ^= 1;
+  FDSP_TRY(launch_polar(reinterpret_cast<const float2*>(d_in), (int64_t)n_in, h->d_prev, h->have_prev ? 0 : 1, d_out,
+                        (cudaStream_t)stream));
   h->have_prev = true;
   return FDSP_OK;
 }

@@ -106,16 +106,16 @@ int launch_cf32_to_ci16(const float2* in, int64_t n, short2* out, cudaStream_t s
 }
 
 // out[i - start] = atan2(Im, Re) of x[i] * conj(x[i-1]); x[-1] is the sample
-// saved by the previous apply (polar_discriminator.cc:150-165).  The last block
-// saves x[N-1] for the next one, into the other of two slots (another block
-// may still read this one's): a launch of its own took 2 us.  Bound by the
-// arc tangent's instructions: a thread's four outputs are independent chains.
+// saved by the previous apply (polar_discriminator.cc:150-165).  The first
+// thread, the only one that reads it, then saves x[N-1] in its place for the
+// next apply (a launch of its own took 2 us; one slot, so that a captured
+// apply carries the state from replay to replay).  Bound by the arc tangent's
+// instructions: a thread's four outputs are independent chains.
 constexpr int kPolarThreads = 256;
 constexpr int kPolarPer = 4;
 
 __global__ void __launch_bounds__(kPolarThreads)
-    polar_kernel(const float2* __restrict__ in, int64_t N, const float2* __restrict__ prev, float2* __restrict__ next,
-                 int start, float* __restrict__ out) {
+    polar_kernel(const float2* __restrict__ in, int64_t N, float2* prev, int start, float* __restrict__ out) {
   grid_dependency();
   const int64_t i0 = (int64_t)blockIdx.x * (kPolarThreads * kPolarPer) + threadIdx.x + start;
   float2 a[kPolarPer], b[kPolarPer];
@@ -131,20 +131,20 @@ __global__ void __launch_bounds__(kPolarThreads)
 #pragma unroll
   for (int u = 0; u < kPolarPer; ++u) {
     const int64_t i = i0 + u * kPolarThreads;
-    // a * conj(b), rounded like the reference's complex<float> product
+    // a * conj(b); the compiler fuses one product into each sum, so an angle's
+    // last bit may differ from a separately rounded product's
     const float re = a[u].x * b[u].x + a[u].y * b[u].y;
     const float im = a[u].y * b[u].x - a[u].x * b[u].y;
     if (i < N) out[i - start] = atan2f(im, re);
   }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *next = in[N - 1];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *prev = in[N - 1];
 }
 
-int launch_polar(const float2* in, int64_t N, const float2* d_prev, float2* d_next, int start, float* out,
-                 cudaStream_t stream) {
+int launch_polar(const float2* in, int64_t N, float2* d_prev, int start, float* out, cudaStream_t stream) {
   if (N <= 0) return FDSP_OK;
   const int64_t per = kPolarThreads * kPolarPer, nblocks = std::max<int64_t>(1, (N - start + per - 1) / per);
   if (nblocks > 0x7fffffffLL) return FDSP_ERR_UNSUPPORTED;
-  void* args[] = {&in, &N, &d_prev, &d_next, &start, &out};
+  void* args[] = {&in, &N, &d_prev, &start, &out};
   return cuda_status(launch_overlapped(reinterpret_cast<const void*>(polar_kernel), dim3((unsigned)nblocks),
                                        dim3(kPolarThreads), 0, stream, args));
 }

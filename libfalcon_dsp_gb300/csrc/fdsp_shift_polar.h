@@ -19,8 +19,7 @@ int launch_freq_shift(const ShiftLaunch& L, cudaStream_t stream);
 // complex64 -> complex int16 by truncation toward zero (the C++ conversion of
 // the reference's int16 overloads)
 int launch_cf32_to_ci16(const float2* in, int64_t n, short2* out, cudaStream_t stream);
-// d_prev: x[-1] of this call (read when start is 0); d_next: where x[N-1] is saved for the next one
-int launch_polar(const float2* in, int64_t N, const float2* d_prev, float2* d_next, int start, float* out,
-                 cudaStream_t stream);
+// d_prev: x[-1] of this call (read when start is 0); afterwards x[N-1], for the next one
+int launch_polar(const float2* in, int64_t N, float2* d_prev, int start, float* out, cudaStream_t stream);
 
 }  // namespace fdsp
