@@ -328,20 +328,33 @@ class MultiRateChannelizerCuda(_Handle):
         return [o[: n_out[i]] for i, o in enumerate(outs)]
 
     def _apply_ci16_device(self, x16, out, stream):
-        return self._enqueue("fdsp_channelizer_apply_ci16", x16, x16.shape[0], out, stream)
+        out, counts, _ = self._enqueue("fdsp_channelizer_apply_ci16", x16, x16.shape[0], out, stream)
+        return [o[:c] for o, c in zip(out, counts)]
 
     def _apply_device(self, x, out, stream):
         x = _dev_c64(x)
-        return self._enqueue("fdsp_channelizer_apply", x, x.numel(), out, stream)
+        out, counts, views = self._enqueue("fdsp_channelizer_apply", x, x.numel(), out, stream)
+        # a channel's count takes two values, so each channel keeps its views
+        # by count (slicing 64 outputs anew took 80 us a call); the handle then
+        # holds the buffers until the next call, as it always did for complex64
+        try:
+            return [v[c] for v, c in zip(views, counts)]
+        except KeyError:
+            for v, o, c in zip(views, out, counts):
+                if c not in v:
+                    if len(v) >= 4:
+                        v.clear()
+                    v[c] = o[:c]
+            return [v[c] for v, c in zip(views, counts)]
 
     def _enqueue(self, fn: str, x, n: int, out, stream):
+        """Runs fn over the output buffers: (the buffers, each one's count,
+        each one's kept views by count)."""
         torch = _torch()
         if out is None:
             out = [torch.empty(max(c, 1), dtype=torch.complex64, device=x.device) for c in self.out_count(n)]
-        # the ctypes arrays and the views of the output buffers are rebuilt
-        # when the caller's buffers change (streaming loops reuse them); a
-        # channel's count takes two values, so each channel keeps its views by
-        # count (slicing 64 outputs anew took 80 us a call)
+        # the ctypes arrays are rebuilt when the caller's buffers change
+        # (streaming loops reuse them)
         ptrs = tuple(map(torch.Tensor.data_ptr, out))
         sizes = tuple(map(torch.Tensor.numel, out))
         oc = getattr(self, "_out_cache", None)
@@ -355,16 +368,7 @@ class MultiRateChannelizerCuda(_Handle):
                                       _stream_handle() if stream is None else stream)
         if st:
             _capi.check(fn, st)
-        counts = n_out[:]
-        try:
-            return [v[c] for v, c in zip(views, counts)]
-        except KeyError:
-            for v, o, c in zip(views, out, counts):
-                if c not in v:
-                    if len(v) >= 4:
-                        v.clear()
-                    v[c] = o[:c]
-            return [v[c] for v, c in zip(views, counts)]
+        return out, n_out[:], views
 
 
 class PolyphaseResamplerCuda(_Handle):
