@@ -34,3 +34,30 @@ def test_int16_apply_keeps_no_output_memory(own):
     gc.collect()
     torch.cuda.synchronize()
     assert torch.cuda.memory_allocated() <= before
+
+
+class _Buffer:
+    """A device buffer that is no tensor: an address and a size."""
+
+    def __init__(self, n):
+        import torch
+        self.t = torch.zeros(n, dtype=torch.complex64, device="cuda")
+
+    def data_ptr(self):
+        return self.t.data_ptr()
+
+    def numel(self):
+        return self.t.numel()
+
+    def __getitem__(self, i):
+        return self.t[i]
+
+
+@pytest.mark.parametrize("dtype", ["c64", "ci16"])
+def test_outputs_may_be_any_object_with_an_address_and_a_size(dtype):
+    import torch
+    x = _ci16(4096) if dtype == "ci16" else torch.randn(4096, dtype=torch.complex64, device="cuda")
+    want = _channelizer().apply(x)
+    got = _channelizer().apply(x, out=[_Buffer(1030) for _ in range(3)])
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
