@@ -69,9 +69,11 @@ def _stream_handle() -> int:
     return _raw_stream(torch.cuda.current_device())
 
 
-def _head(t, n: int):
-    """The first n elements of t: t itself when that is all of it."""
-    return t if t.shape[0] == n else t[:n]
+def _head(t, n: int, given):
+    """The first n elements of t as a view; t itself when that is all of it and
+    the call allocated it (`given`, the caller's output buffer, is None): a
+    caller's buffer is never the result, which may be resized."""
+    return t if given is None and t.shape[0] == n else t[:n]
 
 
 def _c64(x) -> np.ndarray:
@@ -436,6 +438,7 @@ class PolyphaseResamplerCuda(_Handle):
             x = x16 if x16 is not None else _dev_c64(x)
             n_in = x.shape[0] if x16 is not None else x.numel()
             got = C.c_uint64()
+            given = out
             if out is None:
                 st = lib.fdsp_resampler_out_count(self._h, n_in, C.byref(got))
                 if st:
@@ -445,7 +448,7 @@ class PolyphaseResamplerCuda(_Handle):
                                   _stream_handle() if stream is None else stream)
             if st:
                 _capi.check(fn, st)
-            return _head(out, got.value)
+            return _head(out, got.value, given)
         real_in = np.isrealobj(x) and np.asarray(x).dtype != np.int16
         xa = _c64(x)
         n = self.out_count(xa.size)
@@ -494,6 +497,7 @@ class FreqShiftCuda(_Handle):
             torch = _torch()
             x16 = _ci16_dev(x)
             n = x16.shape[0]
+            given = out
             if out is None:
                 out = [torch.empty((max(n, 1), 2), dtype=torch.int16, device=x16.device)
                        for _ in range(self.num_channels)]
@@ -502,7 +506,7 @@ class FreqShiftCuda(_Handle):
                                                         _stream_handle() if stream is None else stream)
             if st:
                 _capi.check("fdsp_freq_shift_apply_ci16", st)
-            res = [_head(o, n) for o in out]
+            res = [_head(o, n, given) for o in out]
             return res[0] if self.single else res
         if not _is_tensor(x) and _ci16_host(x) is not None:
             x16 = _ci16_host(x)
@@ -516,6 +520,7 @@ class FreqShiftCuda(_Handle):
             torch = _torch()
             x = _dev_c64(x)
             n = x.numel()
+            given = out
             if out is None:
                 out = [torch.empty(max(n, 1), dtype=torch.complex64, device=x.device)
                        for _ in range(self.num_channels)]
@@ -524,7 +529,7 @@ class FreqShiftCuda(_Handle):
                                                    _stream_handle() if stream is None else stream)
             if st:
                 _capi.check("fdsp_freq_shift_apply", st)
-            res = [_head(o, n) for o in out]
+            res = [_head(o, n, given) for o in out]
         else:
             xa = _c64(x)
             res = [np.empty(max(xa.size, 1), np.complex64) for _ in range(self.num_channels)]
@@ -572,20 +577,22 @@ class FirFilterCuda(_Handle):
             s = _stream_handle() if stream is None else stream
             if x16 is not None:
                 n = x16.shape[0]
+                given = out
                 if out is None:
                     out = torch.empty((max(n, 1), 2), dtype=torch.int16, device=x16.device)
                 st = _capi.lib().fdsp_fir_apply_ci16(self._h, x16.data_ptr(), n, out.data_ptr(), s)
                 if st:
                     _capi.check("fdsp_fir_apply_ci16", st)
-                return _head(out, n)
+                return _head(out, n, given)
             x = _dev_c64(x)
             n = x.numel()
+            given = out
             if out is None:
                 out = torch.empty(max(n, 1), dtype=torch.complex64, device=x.device)
             st = _capi.lib().fdsp_fir_apply(self._h, x.data_ptr(), n, out.data_ptr(), s)
             if st:
                 _capi.check("fdsp_fir_apply", st)
-            return _head(out, n)
+            return _head(out, n, given)
         x16 = _ci16_host(x)
         if x16 is not None:
             n = x16.shape[0]
@@ -614,6 +621,7 @@ class PolarDiscriminatorCuda(_Handle):
         if _is_tensor(x):
             torch = _torch()
             x = _dev_c64(x)
+            given = out
             if out is None:
                 out = torch.empty(max(x.numel(), 1), dtype=torch.float32, device=x.device)
             got = C.c_uint64()
@@ -621,7 +629,7 @@ class PolarDiscriminatorCuda(_Handle):
                                               _stream_handle() if stream is None else stream)
             if st:
                 _capi.check("fdsp_polar_apply", st)
-            return _head(out, got.value)
+            return _head(out, got.value, given)
         xa = _c64(x)
         y = np.empty(max(xa.size, 1), np.float32)
         got = C.c_uint64()
@@ -679,13 +687,14 @@ class FmDemodulatorCuda(_Handle):
         if _is_tensor(x):
             torch = _torch()
             x = _dev_c64(x)
+            given = out
             if out is None:
                 out = torch.empty(max(n, 1), dtype=torch.int16, device=x.device)
             st = _capi.lib().fdsp_fm_demod_apply(self._h, x.data_ptr(), x.numel(), out.data_ptr(), out.numel(),
                                                  C.byref(got), _stream_handle() if stream is None else stream)
             if st:
                 _capi.check("fdsp_fm_demod_apply", st)
-            return _head(out, got.value)
+            return _head(out, got.value, given)
         xa = _c64(x)
         y = np.empty(max(n, 1), np.int16)
         _capi.call("fdsp_fm_demod_apply_host", self._h, _ptr(xa), xa.size, _ptr(y), y.size, C.byref(got),

@@ -2,6 +2,7 @@
 accepts and what it returns."""
 import gc
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +62,38 @@ def test_outputs_may_be_any_object_with_an_address_and_a_size(dtype):
     got = _channelizer().apply(x, out=[_Buffer(1030) for _ in range(3)])
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+def _calls():
+    import torch
+
+    import libfalcon_dsp_gb300 as F
+    from libfalcon_dsp_gb300.workloads import FM_RADIO_FS, kaiser_lowpass
+    n = 1000
+    c = torch.randn(n, dtype=torch.complex64, device="cuda")
+    c64 = lambda k: torch.empty(k, dtype=torch.complex64, device="cuda")  # noqa: E731
+    i16 = lambda k: torch.empty((k, 2), dtype=torch.int16, device="cuda")  # noqa: E731
+    r = F.PolyphaseResamplerCuda(1, 4, kaiser_lowpass(1, 4, 16))
+    p = F.PolarDiscriminatorCuda()
+    p.apply(c)
+    taps = np.ones(8, np.complex64)
+    d = F.FmDemodulatorCuda(FM_RADIO_FS, 150000)
+    fm = torch.randn(100_000, dtype=torch.complex64, device="cuda")
+    k = F.FmDemodulatorCuda(FM_RADIO_FS, 150000).demod_mono(fm).numel()
+    audio = torch.empty(k, dtype=torch.int16, device="cuda")
+    yield (lambda o: r.apply(c, out=o)), c64(250)
+    yield (lambda o: F.FirFilterCuda(taps).apply(c, out=o)), c64(n)
+    yield (lambda o: F.FirFilterCuda(taps).apply(_ci16(n), out=o)), i16(n)
+    yield (lambda o: F.FreqShiftCuda(1_000_000, 1000).apply(c, out=[o])), c64(n)
+    yield (lambda o: F.FreqShiftCuda(1_000_000, 1000).apply(_ci16(n), out=[o])), i16(n)
+    yield (lambda o: p.apply(c, out=o)), torch.empty(n, dtype=torch.float32, device="cuda")
+    yield (lambda o: d.demod_mono(fm, out=o)), audio
+
+
+def test_a_full_output_is_a_view_of_the_callers_buffer():
+    for call, out in _calls():
+        shape = tuple(out.shape)
+        y = call(out)
+        assert tuple(y.shape) == shape and y.data_ptr() == out.data_ptr() and y is not out
+        y.resize_(1)  # (of the result alone)
+        assert tuple(out.shape) == shape
