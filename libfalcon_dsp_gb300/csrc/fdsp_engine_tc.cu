@@ -1091,40 +1091,26 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
     if (tc_finish(p, (int64_t)n, H_, num_sms_) != 0) return FDSP_ERR_UNSUPPORTED;
   if (plans.empty()) return FDSP_OK;
   if (plans.size() > (size_t)kTcMaxGroups) return FDSP_ERR_UNSUPPORTED;
-  // scratch (grow only): the split input, which every pack reads, and the B
-  // images of every pack (a 1 KB aligned region each)
-  int64_t xhl_need = 0;
-  size_t b_need = 0;
-  std::vector<size_t> boff(plans.size()), ioff(plans.size());
-  size_t i_need = 0;
-  for (size_t li = 0; li < plans.size(); ++li) {
-    ioff[li] = i_need;
-    i_need += (size_t)plans[li].items;
-    xhl_need = std::max(xhl_need, plans[li].xhl_samples);
-    boff[li] = b_need;
-    b_need += (plans[li].b_bytes + 1023u) & ~(size_t)1023u;
-  }
-  if ((size_t)xhl_need > xhl_cap_) {
-    if (d_xhl_) dfree(d_xhl_);
-    d_xhl_ = nullptr;
-    xhl_cap_ = 0;
-    FDSP_TRY(cuda_status(dalloc(reinterpret_cast<void**>(&d_xhl_), (size_t)xhl_need * sizeof(uint2))));
-    xhl_cap_ = (size_t)xhl_need;
-  }
-  if (b_need > bbuf_cap_) {
-    if (d_bbuf_) dfree(d_bbuf_);
-    d_bbuf_ = nullptr;
-    bbuf_cap_ = 0;
-    FDSP_TRY(cuda_status(dalloc(reinterpret_cast<void**>(&d_bbuf_), b_need)));
-    bbuf_cap_ = b_need;
-  }
-  if (i_need > items_cap_) {
-    if (d_items_) dfree(d_items_);
-    d_items_ = nullptr;
-    items_cap_ = 0;
-    FDSP_TRY(cuda_status(dalloc(reinterpret_cast<void**>(&d_items_), i_need * sizeof(uint2))));
-    items_cap_ = i_need;
-  }
+  // scratch (grow only): the split input, which every pack reads, the B images
+  // and the item list of every pack
+  const TcScratch sc = tc_scratch(plans);
+  auto grow = [&](auto** p, size_t* cap, size_t need, size_t slack) {
+    return grow_scratch(
+        p, cap, need, slack,
+        // a pool gives a released range to other engines, on other streams,
+        // while earlier applies queued on this stream may still read it
+        // (without a pool cudaFree waits for them)
+        [&]() { return pool_ ? cuda_status(cudaStreamSynchronize(stream)) : (int)FDSP_OK; },
+        [&](void* q) { dfree(q); },
+        [&](auto** q, size_t n) {
+          const int st = cuda_status(dalloc(reinterpret_cast<void**>(q), n * sizeof(**q)));
+          if (st != FDSP_OK) cudaGetLastError();
+          return st;
+        });
+  };
+  FDSP_TRY(grow(&d_xhl_, &xhl_cap_, sc.xhl, sc.xhl_slack));
+  FDSP_TRY(grow(&d_bbuf_, &bbuf_cap_, sc.b, sc.b_slack));
+  FDSP_TRY(grow(&d_items_, &items_cap_, sc.items, sc.items_slack));
   PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) return FDSP_ERR_UNSUPPORTED;
   // (side streams and events made by build_tc, outside any stream capture)
@@ -1150,12 +1136,12 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
     L.nco = d_nco_;
     L.ctaps = d_ctab_;
     L.xhl = d_xhl_;
-    L.bbuf = d_bbuf_ + boff[li];
+    L.bbuf = d_bbuf_ + sc.b_off[li];
     L.err = d_err_;
     L.rec_out = d_tcrec_ + li;
     L.N = (int64_t)n;
     L.Lc = plan.Lc;
-    L.xhl_n = xhl_need;
+    L.xhl_n = (int64_t)sc.xhl;
     L.H = H_;
     L.G = plan.G;
     L.nmsets = (int32_t)plan.ms.size();
@@ -1180,7 +1166,7 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
       pieces += plan.ms[m].nchunks * 4 * plan.ms[m].NS * 8;
     }
     L.bprefix[plan.ms.size()] = pieces;
-    L.items = d_items_ + ioff[li];
+    L.items = d_items_ + sc.item_off[li];
     int items = 0;
     for (size_t m = 0; m < plan.ms.size(); ++m) {
       L.iprefix[m] = items;
@@ -1213,7 +1199,7 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
     }
     // prep: B images (few blocks), then, for the first launch, the split
     const int nb_build = std::max(1, std::min(num_sms_, (std::max(pieces, items) + 255) / 256));
-    const int64_t nb_split = li == 0 ? std::min<int64_t>((xhl_need + 255) / 256, (int64_t)num_sms_ * 8) : 0;
+    const int64_t nb_split = li == 0 ? std::min<int64_t>(((int64_t)sc.xhl + 255) / 256, (int64_t)num_sms_ * 8) : 0;
     auto prep = tc_fmt_ == 0 ? tc_prep_kernel<0> : tc_prep_kernel<1>;
     int nbb = nb_build;
     cudaError_t e = klaunch(reinterpret_cast<const void*>(prep), dim3((unsigned)(nb_build + nb_split)), dim3(256), 0,

@@ -71,4 +71,28 @@ class RangePool {
   std::map<size_t, size_t> used_;  // offset -> bytes
 };
 
+// Grows a scratch buffer (*p, *cap elements) to at least `need` elements,
+// `slack` more where the memory is there.  The old buffer is released before
+// the new one is allocated, and only after wait() has returned 0: in a pool its
+// range may go to another owner at once, while work queued earlier still reads
+// it.  Returns 0, or the status of the wait() or alloc(p, elements) that failed
+// (after the latter the buffer is empty).
+template <class T, class Wait, class Release, class Alloc>
+int grow_scratch(T** p, size_t* cap, size_t need, size_t slack, Wait wait, Release release, Alloc alloc) {
+  if (need <= *cap) return 0;
+  if (*p) {
+    const int rc = wait();
+    if (rc != 0) return rc;
+    release(*p);
+    *p = nullptr;
+    *cap = 0;
+  }
+  size_t n = need + slack;
+  int rc = alloc(p, n);
+  if (rc != 0 && slack > 0) rc = alloc(p, n = need);
+  if (rc != 0) *p = nullptr;
+  *cap = rc == 0 ? n : 0;
+  return rc;
+}
+
 }  // namespace fdsp

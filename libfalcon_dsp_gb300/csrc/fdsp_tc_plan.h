@@ -534,6 +534,33 @@ inline int tc_finish(TcPlan& p, int64_t N, int H, int num_sms) {
   return 0;
 }
 
+// Scratch of an apply: the split input (samples), the B images (bytes, a 1 KB
+// aligned region per launch) and the item lists (items, one after another).
+// Between blocks of equal size the windows' offsets move; the slack covers a
+// period of the largest row stride and two chunks, two chunks of taps per
+// merge set and an eighth for merge sets that fall another way, and twice the
+// items, so that few streams' buffers grow after their first block.
+struct TcScratch {
+  size_t xhl = 0, b = 0, items = 0;
+  size_t xhl_slack = 0, b_slack = 0, items_slack = 0;
+  std::vector<size_t> b_off, item_off;  // each launch's parts
+};
+inline TcScratch tc_scratch(const std::vector<TcPlan>& plans) {
+  TcScratch s;
+  for (const TcPlan& p : plans) {
+    s.b_off.push_back(s.b);
+    s.item_off.push_back(s.items);
+    s.b += (p.b_bytes + 1023u) & ~(size_t)1023u;
+    s.items += (size_t)p.items;
+    s.xhl = std::max(s.xhl, (size_t)p.xhl_samples);
+    for (const TcPlanGroup& g : p.groups) s.xhl_slack = std::max(s.xhl_slack, (size_t)g.D + 2 * kTcChunkTaps);
+    for (const TcMset& m : p.ms) s.b_slack += 2 * (size_t)tc_round_up((int64_t)4 * m.NS * 128, 1024);
+  }
+  s.b_slack += s.b / 8;
+  s.items_slack = s.items;
+  return s;
+}
+
 // Every group in one launch.  Returns 0 on success, -1 when they exceed a
 // launch's record limits.
 inline int tc_plan(const std::vector<TcGroupIn>& gin, int64_t N, int H, int num_sms, TcPlan& p) {
