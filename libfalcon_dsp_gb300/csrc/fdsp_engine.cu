@@ -84,18 +84,22 @@ __device__ __forceinline__ float2 unpack2(f32x2 v) {
 
 // kRows rows (jl, jl + 32, ...) of one work set with NB live channels: T
 // complex MACs per row and channel (taps and samples from shared memory), then
-// rotation and store.  Taps are stored [T][NB] as (re, re, im, im), so a
+// rotation and store.  Packed taps are stored [T][NB] as (re, re, im, im), so a
 // complex MAC is two packed multiply-adds of the sample as it lies in memory:
 // a += (re, re) x, b += (im, im) x, and the output is (a.x - b.y, a.y + b.x).
+// Compact taps (re, im) take half the room and the same multiply-adds one
+// component at a time (packed ones too where four rows share the copies).
 // Bound: issue slots and shared-memory reads.  A tap read (a broadcast) feeds
 // kRows samples, a sample read NB channels.  Sums run over the taps in order
 // whatever kRows is, so an output's bits do not depend on the tile height.
-template <int NB, int kRows>
+template <int NB, int kRows, bool kPacked>
 __device__ __forceinline__ void process_rows(const float2* __restrict__ xs, const float4* __restrict__ tp,
                                              const ChanMeta* __restrict__ meta, int T, int D, int P, int nph, int b0,
                                              int q0, int64_t j, int64_t J, int U, int r, int delta) {
   const f32x2* xp = reinterpret_cast<const f32x2*>(xs + b0 * P + q0);
+  constexpr int kPitch = (NB + 1) & ~1;  // compact taps of a row
   const ulonglong2* tq = reinterpret_cast<const ulonglong2*>(tp);
+  const float2* tc = reinterpret_cast<const float2*>(tp);
   const int wrap = 1 - nph * P;
   f32x2 sa[kRows][NB], sb[kRows][NB];
 #pragma unroll
@@ -109,17 +113,45 @@ __device__ __forceinline__ void process_rows(const float2* __restrict__ xs, cons
       f32x2 x[kRows];
 #pragma unroll
       for (int q = 0; q < kRows; ++q) x[q] = xp[32 * q];
+      if constexpr (kPacked) {
 #pragma unroll
-      for (int n = 0; n < NB; ++n) {
-        const ulonglong2 g = tq[n];
+        for (int n = 0; n < NB; ++n) {
+          const ulonglong2 g = tq[n];
 #pragma unroll
-        for (int q = 0; q < kRows; ++q) {
-          sa[q][n] = fma2(g.x, x[q], sa[q][n]);
-          sb[q][n] = fma2(g.y, x[q], sb[q][n]);
+          for (int q = 0; q < kRows; ++q) {
+            sa[q][n] = fma2(g.x, x[q], sa[q][n]);
+            sb[q][n] = fma2(g.y, x[q], sb[q][n]);
+          }
         }
+        tq += NB;
+      } else {
+        float2 g[kPitch];
+#pragma unroll
+        for (int n = 0; n < NB; n += 2) {
+          if (n + 1 < NB) {
+            const float4 v = *reinterpret_cast<const float4*>(tc + n);
+            g[n] = make_float2(v.x, v.y);
+            g[n + 1] = make_float2(v.z, v.w);
+          } else {
+            g[n] = tc[n];
+          }
+        }
+#pragma unroll
+        for (int n = 0; n < NB; ++n)
+#pragma unroll
+          for (int q = 0; q < kRows; ++q) {
+            if constexpr (kRows >= 4) {
+              sa[q][n] = fma2(pack2(g[n].x, g[n].x), x[q], sa[q][n]);
+              sb[q][n] = fma2(pack2(g[n].y, g[n].y), x[q], sb[q][n]);
+            } else {
+              const float2 v = unpack2(x[q]), a = unpack2(sa[q][n]), b = unpack2(sb[q][n]);
+              sa[q][n] = pack2(fmaf(g[n].x, v.x, a.x), fmaf(g[n].x, v.y, a.y));
+              sb[q][n] = pack2(fmaf(g[n].y, v.x, b.x), fmaf(g[n].y, v.y, b.y));
+            }
+          }
+        tc += kPitch;
       }
       xp += P;
-      tq += NB;
     }
   }
 
@@ -175,8 +207,13 @@ __device__ __forceinline__ void process_rows(const float2* __restrict__ xs, cons
       qq += q0 + 32 * q;
       for (int k = er.k0; k < T; ++k) {
         const float2 x = xs[bb * P + qq];
-        const float4 g4 = tp[k * NB + n];
-        const float2 gk = make_float2(g4.x, g4.z);
+        float2 gk;
+        if constexpr (kPacked) {
+          const float4 g4 = tp[k * NB + n];
+          gk = make_float2(g4.x, g4.z);
+        } else {
+          gk = reinterpret_cast<const float2*>(tp)[k * kPitch + n];
+        }
         B.x = fmaf(gk.x, x.x, B.x);
         B.x = fmaf(-gk.y, x.y, B.x);
         B.y = fmaf(gk.x, x.y, B.y);
@@ -194,16 +231,16 @@ __device__ __forceinline__ void process_rows(const float2* __restrict__ xs, cons
 
 // The row blocks of one work set: two rows a thread where the tile height
 // allows (four in engines of one or two channels a batch), one otherwise.
-template <int NB>
+template <int NB, bool kPacked>
 __device__ __forceinline__ void process_block(int rows, const float2* __restrict__ xs, const float4* __restrict__ tp,
                                               const ChanMeta* __restrict__ meta, int T, int D, int P, int nph, int b0,
                                               int q0, int64_t j, int64_t J, int U, int r, int delta) {
   if (NB <= 2 && rows == 4) {
-    process_rows<NB, NB <= 2 ? 4 : 2>(xs, tp, meta, T, D, P, nph, b0, q0, j, J, U, r, delta);
+    process_rows<NB, NB <= 2 ? 4 : 2, kPacked>(xs, tp, meta, T, D, P, nph, b0, q0, j, J, U, r, delta);
   } else if (rows >= 2) {
-    process_rows<NB, 2>(xs, tp, meta, T, D, P, nph, b0, q0, j, J, U, r, delta);
+    process_rows<NB, 2, kPacked>(xs, tp, meta, T, D, P, nph, b0, q0, j, J, U, r, delta);
   } else {
-    process_rows<NB, 1>(xs, tp, meta, T, D, P, nph, b0, q0, j, J, U, r, delta);
+    process_rows<NB, 1, kPacked>(xs, tp, meta, T, D, P, nph, b0, q0, j, J, U, r, delta);
   }
 }
 
@@ -221,6 +258,9 @@ constexpr int kWinRows = 7;
 // Shared memory of a CTA that leaves room for two more, or one more, on the SM.
 constexpr int kSmem3 = 75 * 1024;
 constexpr int kSmem2 = 112 * 1024;
+// Taps are staged while the CTA stays within this; longer filters of many
+// phases read them through L1.
+constexpr int kSmemTaps = 150 * 1024;
 
 // Rotation and store of one single-channel output (the per-row epilogue
 // for NB = 1).
@@ -363,7 +403,7 @@ __device__ __forceinline__ void hist_sample(const float2* __restrict__ old_hist,
 // launch's groups (fuse_map[first ..]) follow one another in blockIdx.x, and
 // the blocks past the last tile write the history of the next block.  Shared
 // memory: [input tile, de-interleaved: nph x P float2][taps of every work set
-// of the group, packed [T][nb]][ChanMeta per (work set, channel)].
+// of the group][ChanMeta per (work set, channel)].
 //
 // One launch over all groups: a group alone has 100-400 tiles, 1-2 a SM, so
 // launches one after another each ended in a nearly empty wave (64 channels of
@@ -373,7 +413,7 @@ __device__ __forceinline__ void hist_sample(const float2* __restrict__ old_hist,
 // windows overlap or wrap, else (long decimations) only the groups' windows,
 // up to kMaxSegs segments of them (seg_at / seg_gap map a staged phase to its
 // place in the row).
-template <int NBMAX, bool kTapsSmem, bool kWin>
+template <int NBMAX, int kTaps, bool kWin>
 __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
     poly_fp32_kernel(const __grid_constant__ PolyLaunch<NBMAX> L, int first, int tiles) {
   extern __shared__ __align__(16) float2 xs[];
@@ -483,8 +523,8 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
   // after another with plain loads took a memory latency each).
   for (int wi = warp; wi < nws; wi += kThreads / 32) {
     const WorkSet<NBMAX>& W = L.ws[G.ws_begin + wi];
-    if constexpr (kTapsSmem) {
-      const int cnt = W.T * W.nb;
+    if constexpr (kTaps != kTapsGlobal) {
+      const int cnt = kTaps == kTapsPacked ? W.T * W.nb : W.T * ((W.nb + 1) >> 1);
       const float4* src = W.taps;
       const uint32_t dst = (uint32_t)__cvta_generic_to_shared(taps_s + W.soff);
       for (int i = lane; i < cnt; i += 32)
@@ -528,7 +568,7 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
       const bool mine = wq < nws && row0 + jl0 < W.J;
       if (mine) {
         const int a0 = (W.delta - G.delta_min) + (G.tmax - W.T);
-        const float4* tp = kTapsSmem ? taps_s + W.soff : W.taps;
+        const float4* tp = kTaps != kTapsGlobal ? taps_s + W.soff : W.taps;
         if (G.real_taps)
           win_sums<true>(xs, tp, W.T, D, P, a0, jl0, acc);
         else
@@ -554,7 +594,7 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
       if (j0 >= W.J) continue;
       const int T = W.T;
       const int a0 = (W.delta - G.delta_min) + (G.tmax - T);
-      const float4* tp = kTapsSmem ? taps_s + W.soff : W.taps;
+      const float4* tp = kTaps != kTapsGlobal ? taps_s + W.soff : W.taps;
       const ChanMeta* mt = meta_s + wq * NBMAX;
       if (G.real_taps)
         win_sums<true>(xs, tp, T, D, P, a0, jl0, acc);
@@ -580,12 +620,12 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
     if (row0 + jl >= W.J) continue;
     const int64_t j = row0 + jl + lane;
     const int T = W.T, b0 = W.b0, q0 = W.q0 + jl + lane;
-    const float4* tp = kTapsSmem ? taps_s + W.soff : W.taps;
+    const float4* tp = kTaps != kTapsGlobal ? taps_s + W.soff : W.taps;
     const ChanMeta* mt = meta_s + wq * NBMAX;
 #define FDSP_NB(n)                                                                                        \
   case n:                                                                                                 \
     if constexpr (NBMAX >= n)                                                                             \
-      process_block<n>(rows, xs, tp, mt, T, D, P, nph, b0, q0, j, (int64_t)W.J, W.U, W.r, W.delta);       \
+      process_block<n, kTaps == kTapsPacked>(rows, xs, tp, mt, T, D, P, nph, b0, q0, j, (int64_t)W.J, W.U, W.r, W.delta);       \
     break;
     switch (W.nb) {
       FDSP_NB(1)
@@ -972,11 +1012,14 @@ int PolyEngine::init(uint32_t fs, const fdsp_channel_cfg* ch, uint32_t nch, bool
     }
   }
 
-  // modulated, padded taps of every batch: [up][T][channels] as (re, re, im, im)
+  // modulated, padded taps of every batch: [up][T][channels] as (re, re, im,
+  // im), then as (re, im) with the channels padded to an even number
   for (auto& bt : batches_) {
     const uint32_t U = classes_[bt.cls].up;
     const size_t nb = bt.chans.size();
-    std::vector<float4> host((size_t)U * bt.T * nb, make_float4(0.f, 0.f, 0.f, 0.f));
+    const size_t packed = (size_t)U * bt.T * nb, pitch = (nb + 1) & ~(size_t)1;
+    std::vector<float4> host(packed + (size_t)U * bt.T * pitch / 2, make_float4(0.f, 0.f, 0.f, 0.f));
+    float2* const compact = reinterpret_cast<float2*>(host.data() + packed);
     for (size_t n = 0; n < bt.chans.size(); ++n) {
       const EngineChannel& e = chans_[bt.chans[n]];
       const int pad = bt.T - (int)e.T;
@@ -998,6 +1041,7 @@ int PolyEngine::init(uint32_t fs, const fdsp_channel_cfg* ch, uint32_t nch, bool
             gi = (double)h.x * s + (double)h.y * c;
           }
           host[((size_t)ph * bt.T + k) * nb + n] = make_float4((float)gr, (float)gr, (float)gi, (float)gi);
+          compact[((size_t)ph * bt.T + k) * pitch + n] = make_float2((float)gr, (float)gi);
         }
       }
     }
@@ -1323,16 +1367,22 @@ static void layout_group(PolyLaunch<NB>& L, GroupDesc& gd, int Qt) {
   int64_t off = ((int64_t)gd.nph * P + 1) & ~1LL;  // float2 units, 16-byte aligned
   if (gd.lines) off = std::max(off, (int64_t)Qt * (gd.ws_end - gd.ws_begin));  // the tile's outputs take its place
   gd.taps_off = (int32_t)off;
+  const int64_t meta_bytes = (int64_t)(gd.ws_end - gd.ws_begin) * NB * 48;
+  int64_t packed = 0, compact = 0;  // float4
+  for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) {
+    packed += (int64_t)L.ws[wi].T * L.ws[wi].nb;
+    compact += (int64_t)L.ws[wi].T * ((L.ws[wi].nb + 1) >> 1);
+  }
+  auto bytes = [&](int64_t taps) { return (off + 2 * taps) * (int64_t)sizeof(float2) + meta_bytes; };
+  auto ctas = [&](int64_t b) { return b <= kSmem3 ? 3 : b <= kSmem2 ? 2 : b <= kSmemTaps ? 1 : 0; };
+  gd.taps = ctas(bytes(packed)) > 0 ? kTapsPacked : kTapsGlobal;
+  if (!gd.win && ctas(bytes(compact)) > ctas(bytes(packed))) gd.taps = kTapsCompact;
   int64_t toff = 0;
   for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) {
     L.ws[wi].soff = (int32_t)toff;
-    toff += (int64_t)L.ws[wi].T * L.ws[wi].nb;
+    toff += (int64_t)L.ws[wi].T * (gd.taps == kTapsPacked ? L.ws[wi].nb : (L.ws[wi].nb + 1) >> 1);
   }
-  const int64_t meta_bytes = (int64_t)(gd.ws_end - gd.ws_begin) * NB * 48;
-  // taps go to shared memory unless they would push the CTA past ~150 KB
-  // (long filters of many phases); those groups read taps through L1
-  gd.taps_smem = ((off + 2 * toff) * (int64_t)sizeof(float2) + meta_bytes <= 150 * 1024) ? 1 : 0;
-  if (gd.taps_smem) off += 2 * toff;
+  if (gd.taps != kTapsGlobal) off += 2 * toff;
   gd.meta_off = (int32_t)off;
   gd.smem_bytes = (int32_t)(off * (int64_t)sizeof(float2) + meta_bytes);
 }
@@ -1363,6 +1413,7 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
   int64_t rows_of[kMaxGroups];
   int qt_of[kMaxGroups];
   bool fixed_qt[kMaxGroups];
+  const float4* compact_of[kMaxWorkSets];  // the work sets' compact taps
   for (auto& g : groups_) {
     GroupDesc& gd = L.groups[ng];
     gd.D = (int32_t)g.D;
@@ -1382,6 +1433,7 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
         if (nws >= kMaxWorkSets) return FDSP_ERR_UNSUPPORTED;
         WorkSet<NB>& W = L.ws[nws++];
         W.taps = bt.d_taps + (size_t)phi * bt.T * bt.chans.size();
+        compact_of[nws - 1] = bt.d_taps + (size_t)U * bt.T * bt.chans.size() + (size_t)phi * bt.T * ((bt.chans.size() + 1) / 2);
         W.T = bt.T;
         W.delta = (int32_t)delta;
         W.J = (int32_t)J;
@@ -1446,6 +1498,8 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
       qt_of[gi] -= 32;
     }
     gd.ntiles = (int32_t)((rows_of[gi] + gd.Qt - 1) / gd.Qt);
+    if (!gd.win && gd.taps != kTapsPacked)
+      for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) L.ws[wi].taps = compact_of[wi];
   }
   // tensor-core groups: one prep launch and one filter-bank launch for all of
   // them; groups the tensor-core plan cannot hold stay on the FP32 kernel
@@ -1467,8 +1521,8 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
   }
   if (d_nat_ && ng == 1 && !on_tc[0] && prof_ev_.empty())
     return launch_nat(d_in, n, out[0], L.groups[0].win == 0, stream);
-  // The FP32 groups in one launch per kernel variant (taps staged or read
-  // through L1, sliding window or rows) and shared-memory size (three CTAs an
+  // The FP32 groups in one launch per kernel variant (how the taps lie,
+  // sliding window or rows) and shared-memory size (three CTAs an
   // SM or fewer), tallest work first; the last launch also writes the history.
   // Group by group only for the autotuner, and for blocks of several waves
   // whose outputs are copied back as groups finish (apply_host).
@@ -1492,20 +1546,24 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
     }
     std::sort(order, order + nfp, [&](int a, int b) { return cost[a] != cost[b] ? cost[a] > cost[b] : a < b; });
     const bool single = !prof_ev_.empty() || (done_fn_ && tiles > 3LL * num_sms_);
-    for (int variant = 0; variant < 12; ++variant) {
-      const bool smem_taps = (variant & 1) == 0, win = (variant & 2) != 0;
-      const int size = variant >> 2;  // CTAs that fit an SM: three or more, two, one
+    const void* const kernels[5] = {reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsPacked, false>),
+                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsCompact, false>),
+                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsGlobal, false>),
+                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsPacked, true>),
+                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsGlobal, true>)};
+    const int taps_of[5] = {kTapsPacked, kTapsCompact, kTapsGlobal, kTapsPacked, kTapsGlobal};
+    for (int variant = 0; variant < 15; ++variant) {
+      const int kind = variant % 5;
+      const int size = variant / 5;  // CTAs that fit an SM: three or more, two, one
       bool open = false;
       for (int i = 0; i < nfp; ++i) {
         const GroupDesc& gd = L.groups[order[i]];
-        if ((gd.taps_smem != 0) != smem_taps || (gd.win != 0) != win || (gd.smem_bytes > kSmem3) + (gd.smem_bytes > kSmem2) != size)
+        if (gd.taps != taps_of[kind] || (gd.win != 0) != (kind >= 3) ||
+            (gd.smem_bytes > kSmem3) + (gd.smem_bytes > kSmem2) != size)
           continue;
         if (!open || single) {
           Batch& nb = lb[nlb++];
-          nb.kern = win ? (smem_taps ? reinterpret_cast<const void*>(poly_fp32_kernel<NB, true, true>)
-                                     : reinterpret_cast<const void*>(poly_fp32_kernel<NB, false, true>))
-                        : (smem_taps ? reinterpret_cast<const void*>(poly_fp32_kernel<NB, true, false>)
-                                     : reinterpret_cast<const void*>(poly_fp32_kernel<NB, false, false>));
+          nb.kern = kernels[kind];
           nb.first = nm;
           nb.count = nb.tiles = 0;
           nb.smem = 0;

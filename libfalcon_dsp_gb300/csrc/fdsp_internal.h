@@ -50,6 +50,11 @@ struct NcoConst {
 // One decimation-factor group of an engine launch (one CTA per tile of it).
 constexpr int kMaxSegs = 4;  // runs of staged phases a row may have
 
+// Taps of a work set: packed as (re, re, im, im) in shared memory; compact as
+// (re, im) in shared memory, rows padded to an even width; or read through L1
+// (compact; the sliding-window form reads packed ones).
+constexpr int kTapsGlobal = 0, kTapsPacked = 1, kTapsCompact = 2;
+
 struct GroupDesc {
   int32_t D;          // down rate shared by every channel of the group
   int32_t Qt;         // output rows per tile (multiple of 32)
@@ -63,7 +68,7 @@ struct GroupDesc {
   int32_t taps_off;   // shared-memory offset (float2) of the staged taps
   int32_t meta_off;   // shared-memory offset (float2) of the staged channel constants
   int32_t smem_bytes; // dynamic shared memory of one CTA
-  int32_t taps_smem;  // 1: taps staged in shared memory; 0: read through L1
+  int32_t taps;       // kTapsPacked .. kTapsGlobal: where and how the taps lie
   int32_t win;        // 1: single-channel work sets, sliding-window rows (Qt multiple of 32 x kWinRows)
   int32_t real_taps;  // 1: every tap of the group is real (2 FMAs per tap)
   int32_t rows;       // rows a thread computes in the row form (1, 2 or 4; Qt is a multiple of 32 rows)
@@ -84,7 +89,7 @@ struct GroupDesc {
 // [delta + j*D - T + 1, delta + j*D] in block-relative input indices.
 template <int NB>
 struct WorkSet {
-  const float4* taps;   // [T][nb] modulated taps of phase phi_r, (re, re, im, im) (device)
+  const float4* taps;   // [T][nb] modulated taps of phase phi_r (device), packed or compact as the group's kernel reads them
   int32_t T;            // padded taps per phase of the batch
   int32_t soff;         // offset (float4) of these taps in the CTA's staged taps
   int32_t delta;        // window end of row j = 0 (block relative)
@@ -277,7 +282,7 @@ struct EngineBatch {
   int group;           // decimation group index
   int T;               // padded taps per phase
   std::vector<int> chans;
-  float4* d_taps;      // [up][T][nb] on the device, (re, re, im, im)
+  float4* d_taps;      // on the device: packed [up][T][nb], then compact [up][T][nb rounded up to even]
 };
 
 struct EngineGroup {
