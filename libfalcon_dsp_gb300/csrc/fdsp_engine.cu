@@ -1489,13 +1489,30 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
   }
   for (int gi = 0; gi < ng; ++gi) {
     GroupDesc& gd = L.groups[gi];
-    for (;;) {  // a lower tile where this one's samples leave no room for the other CTAs (or it is over the limit)
-      layout_group<NB>(L, gd, qt_of[gi]);
-      const int roomy = NB == 8 ? kSmem2 : kSmem3;  // (registers allow two CTAs of 8-channel batches, three of others)
-      const bool trim = !fixed_qt[gi] && gd.smem_bytes > roomy && 16 * (int64_t)gd.taps_off > gd.smem_bytes;
-      if (gd.smem_bytes <= 227 * 1024 && (!trim || qt_of[gi] <= 32)) break;
-      if (gd.win || qt_of[gi] <= 32) return FDSP_ERR_UNSUPPORTED;
-      qt_of[gi] -= 32;
+    const int qt0 = qt_of[gi], nsets = gd.ws_end - gd.ws_begin;
+    layout_group<NB>(L, gd, qt0);
+    // A lower tile where this one's samples leave no room for two more CTAs on
+    // the SM, or one more, and a lower one does: not below one that stages as
+    // much halo as rows or leaves a warp without rows (9700 taps of two
+    // channels over 2^20 samples: 211 ms with 32 rows, 8.3 with 4096)
+    if (!fixed_qt[gi] && 16 * (int64_t)gd.taps_off > gd.smem_bytes) {
+      const int64_t halo = (int64_t)gd.tmax + gd.delta_span;
+      const int base = std::max(32, (4096 / gd.D) & ~31);
+      // (registers allow two CTAs of 8-channel batches, three of others)
+      for (int room : {NB == 8 ? kSmem2 : kSmem3, kSmem2}) {
+        for (int q = qt0 - 32; gd.smem_bytes > room; q -= 32) {
+          if (q < 32 || (q < base && ((int64_t)q * gd.D < halo || nsets * q < kThreads))) {
+            layout_group<NB>(L, gd, qt0);
+            break;
+          }
+          layout_group<NB>(L, gd, q);
+        }
+        if (gd.smem_bytes <= room) break;
+      }
+    }
+    while (gd.smem_bytes > 227 * 1024) {
+      if (gd.win || gd.Qt <= 32) return FDSP_ERR_UNSUPPORTED;
+      layout_group<NB>(L, gd, gd.Qt - 32);
     }
     gd.ntiles = (int32_t)((rows_of[gi] + gd.Qt - 1) / gd.Qt);
     if (!gd.win && gd.taps != kTapsPacked)

@@ -94,6 +94,8 @@ def _time(nch, d, t, n):
 
 
 @pytest.mark.parametrize("nch,d,short,long,n,slack", [
+    (2, 1, 4600, 9700, 1 << 19, 3.5),    # tiles of 32 rows under a halo of 9699 samples took 18 times as long
+    (2, 1, 3000, 5500, 1 << 19, 3.5),
     (4, 10, 1250, 2500, 1 << 21, 1.5),   # taps of twice the size no longer fitted shared memory: 4 times as long
     (8, 10, 600, 1200, 1 << 21, 1.5),
 ])
