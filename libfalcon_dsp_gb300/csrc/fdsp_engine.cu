@@ -296,9 +296,11 @@ constexpr int kWinRows = 7;
 // Shared memory of a CTA that leaves room for two more, or one more, on the SM.
 constexpr int kSmem3 = 75 * 1024;
 constexpr int kSmem2 = 112 * 1024;
-// Taps are staged while the CTA stays within this; longer filters of many
-// phases read them through L1.
-constexpr int kSmemTaps = 150 * 1024;
+// Taps are staged while the CTA stays within this, the SM's limit; longer
+// filters of many phases read them through L1, of which the tile leaves little
+// (3000 taps of four channels by 100 over 2^22 samples: 0.80 ms so, 0.41
+// staged, one CTA an SM).
+constexpr int kSmemTaps = 227 * 1024;
 
 // Rotation and store of one single-channel output (the per-row epilogue
 // for NB = 1).
@@ -1327,7 +1329,6 @@ template <int NB>
 static void layout_group(PolyLaunch<NB>& L, GroupDesc& gd, int Qt) {
   const int D = gd.D;
   gd.Qt = Qt;
-  gd.rows = NB <= 2 && Qt % 128 == 0 ? 4 : Qt % 64 == 0 ? 2 : 1;
   gd.nph = D;
   for (int i = 0; i < kMaxSegs - 1; ++i) {
     gd.seg_at[i] = INT32_MAX;
@@ -1413,8 +1414,15 @@ static void layout_group(PolyLaunch<NB>& L, GroupDesc& gd, int Qt) {
   }
   auto bytes = [&](int64_t taps) { return (off + 2 * taps) * (int64_t)sizeof(float2) + meta_bytes; };
   auto ctas = [&](int64_t b) { return b <= kSmem3 ? 3 : b <= kSmem2 ? 2 : b <= kSmemTaps ? 1 : 0; };
+  // Packed taps take fewer instructions; compact ones where the SM then holds
+  // more CTAs or only one packed one, and for wide batches of short runs, whose
+  // reads bound the kernel (64 taps of 16 channels by 3 over 2^20 samples: 137
+  // us packed, 122 compact; by 10: 43 and 53).
   gd.taps = ctas(bytes(packed)) > 0 ? kTapsPacked : kTapsGlobal;
-  if (!gd.win && ctas(bytes(compact)) > ctas(bytes(packed))) gd.taps = kTapsCompact;
+  if (!gd.win && ctas(bytes(compact)) > 0 &&
+      (ctas(bytes(packed)) <= 1 || ctas(bytes(compact)) > ctas(bytes(packed)) ||
+       (NB >= 4 && gd.nph > 1 && gd.nph <= kShortRun)))
+    gd.taps = kTapsCompact;
   int64_t toff = 0;
   for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) {
     L.ws[wi].soff = (int32_t)toff;
@@ -1423,6 +1431,34 @@ static void layout_group(PolyLaunch<NB>& L, GroupDesc& gd, int Qt) {
   if (gd.taps != kTapsGlobal) off += 2 * toff;
   gd.meta_off = (int32_t)off;
   gd.smem_bytes = (int32_t)(off * (int64_t)sizeof(float2) + meta_bytes);
+  // Rows a thread.  A warp's item takes the instructions of a tap: a sample
+  // read a row, the tap reads, the multiply-adds (packed taps, and four rows
+  // that share the copies, two components at a time) and the walk.  A tile
+  // takes the SM's issue slots for all of its items, or, where its warps are
+  // few, their rounds at one instruction in three cycles a warp (9000 taps of
+  // two channels by 10 over 2^22 samples: 7.2 ms with a row a thread, 4.2 with
+  // two; 300 taps by 6 over 2^20: 68 us and 47).
+  const int ctas_sm = std::max(1, std::min(ctas(gd.smem_bytes), NB == 8 ? 2 : 3)), warps = kThreads / 32;
+  double best_time = 0;
+  for (int r = NB <= 2 ? 4 : 2; r >= 1 && !gd.win; r /= 2) {
+    if (Qt % (32 * r) != 0) continue;
+    int items = 0;
+    double work = 0, cost = 0;
+    for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) {
+      const int nb = L.ws[wi].nb, n = Qt / (32 * r);
+      const bool packed_taps = gd.taps == kTapsPacked;
+      const int tap = r + (packed_taps ? nb : (nb + 1) / 2) + 3 +
+                      (packed_taps ? 2 * nb * r : r >= 4 ? 2 * nb * r + 4 * nb : 4 * nb * r);
+      items += n;
+      work += (double)n * L.ws[wi].T * tap;
+      cost = std::max(cost, (double)L.ws[wi].T * tap);
+    }
+    const double time = std::max(work / 4, (items + warps - 1) / warps * cost * 3 / ctas_sm);
+    if (best_time == 0 || time < best_time) {
+      best_time = time;
+      gd.rows = r;
+    }
+  }
 }
 
 template <int NB>
