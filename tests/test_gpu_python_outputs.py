@@ -29,12 +29,36 @@ def test_int16_apply_keeps_no_output_memory(own):
     torch.cuda.synchronize()
     before = torch.cuda.memory_allocated()
     out = [torch.empty((1 << 18) + 1, dtype=torch.complex64, device="cuda") for _ in range(3)] if own else None
-    res = h.apply(x, out=out)
+    for _ in range(3):
+        res = h.apply(x, out=out)
     assert [r.numel() for r in res] == [1 << 18] * 3 and torch.cuda.memory_allocated() > before
     del res, out
     gc.collect()
     torch.cuda.synchronize()
     assert torch.cuda.memory_allocated() <= before
+
+
+def test_int16_results_follow_the_callers_buffers():
+    import torch
+    x, want = _ci16(4001), []
+    h, f = _channelizer(), _channelizer()
+    for _ in range(9):  # counts of 1000 and 1001, new buffers after three calls, other ones over the same memory
+        want.append([y.clone() for y in f.apply(x)])
+    mem = [torch.zeros(2 * 1040, dtype=torch.complex64, device="cuda") for _ in range(3)]
+    sets = [[m[:1024] for m in mem], [m[5:1030] for m in mem], [m[:1024] for m in mem]]
+    for k in range(9):
+        out = sets[k // 3]
+        for m in mem:
+            m.zero_()
+        got = h.apply(x, out=out)
+        for a, b, o in zip(got, want[k], out):
+            assert torch.equal(a, b) and a.data_ptr() == o.data_ptr() and torch.equal(o[:a.numel()], b)
+    kept = h.apply(x, out=sets[2])
+    again = [t.clone() for t in kept]
+    del sets, out, mem, got
+    gc.collect()
+    torch.randn(1 << 16, device="cuda")  # (the results keep their memory when the buffers go)
+    assert all(torch.equal(a, b) for a, b in zip(kept, again))
 
 
 class _Buffer:
