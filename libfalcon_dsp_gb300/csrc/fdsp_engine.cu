@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
 }
 
 // Rational resampling of one unshifted channel with many output phases
-// (U >= kNatMinUp): consecutive outputs on consecutive lanes.  Their windows
+// (kNatMinUp to kNatMaxUp): consecutive outputs on consecutive lanes.  Their windows
 // start D / U samples apart, so sample reads of the tile as it lies in memory
 // hardly conflict, the taps lie in output order (column r of [T][U]: phase r D
 // mod U; conflict-free, staged as they lie), and stores are contiguous.  The row form gives each of the U phases its own work
@@ -695,6 +695,7 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
 // kCheck keeps that form's products with the taps' zero imaginary parts: an
 // infinite or NaN sample then marks both parts of an output, as it did there.
 constexpr int kNatMinUp = 16;
+constexpr int kNatMaxUp = kMaxWorkSets;  // an apply builds a work set per phase first, and refuses more
 constexpr int kNatMaxTaps = 8192;  // U T: 32 KB of taps in shared memory
 constexpr int kNatPer = 4;         // outputs a thread of a full tile
 constexpr int kNatMaxCols = 512;   // threads of a CTA: a multiple of U columns, rounded up to warps
@@ -1100,8 +1101,8 @@ int PolyEngine::init(uint32_t fs, const fdsp_channel_cfg* ch, uint32_t nch, bool
     r = g0 % b;
     g0 = b;
   }
-  if (nch == 1 && !complex_taps && !chans_[0].nco.enabled && U0 >= (uint32_t)kNatMinUp && U0 <= (uint32_t)kNatMaxCols && g0 == 1 && D0 <= 4u * U0 &&
-      (uint64_t)U0 * chans_[0].T <= (uint64_t)kNatMaxTaps) {
+  if (nch == 1 && !complex_taps && !chans_[0].nco.enabled && U0 >= (uint32_t)kNatMinUp && U0 <= (uint32_t)kNatMaxUp && g0 == 1 &&
+      D0 <= 4u * U0 && (uint64_t)U0 * chans_[0].T <= (uint64_t)kNatMaxTaps) {
     const uint32_t T0 = chans_[0].T;
     std::vector<float> host(((size_t)U0 * T0 + 3) & ~(size_t)3, 0.f);
     nat_col_.assign(U0, 0);
