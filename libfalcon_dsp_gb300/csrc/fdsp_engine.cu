@@ -301,6 +301,8 @@ constexpr int kSmem2 = 112 * 1024;
 // (3000 taps of four channels by 100 over 2^22 samples: 0.80 ms so, 0.41
 // staged, one CTA an SM).
 constexpr int kSmemTaps = 227 * 1024;
+// Complex multiply-adds that a launch of their own pays for (about 60 us).
+constexpr int64_t kSplitWork = 1 << 28;
 
 // Rotation and store of one single-channel output (the per-row epilogue
 // for NB = 1).
@@ -1325,9 +1327,10 @@ void PolyEngine::reset() {
 }
 
 // Tile of Qt rows of one group: which input phases it stages, its pitch, and
-// its shared-memory layout.
+// its shared-memory layout.  keep_packed: packed taps wherever they fit.
+// Returns whether they do.
 template <int NB>
-static void layout_group(PolyLaunch<NB>& L, GroupDesc& gd, int Qt) {
+static bool layout_group(PolyLaunch<NB>& L, GroupDesc& gd, int Qt, bool keep_packed = false) {
   const int D = gd.D;
   gd.Qt = Qt;
   gd.nph = D;
@@ -1408,10 +1411,17 @@ static void layout_group(PolyLaunch<NB>& L, GroupDesc& gd, int Qt) {
   if (gd.lines) off = std::max(off, (int64_t)Qt * (gd.ws_end - gd.ws_begin));  // the tile's outputs take its place
   gd.taps_off = (int32_t)off;
   const int64_t meta_bytes = (int64_t)(gd.ws_end - gd.ws_begin) * NB * 48;
-  int64_t packed = 0, compact = 0;  // float4
+  int64_t packed = 0, compact = 0, tsum = 0;  // taps of all work sets: float4 packed, compact; taps of a channel each
+  int long_t = 0, long_nb = 0;                // the longest work set
   for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) {
-    packed += (int64_t)L.ws[wi].T * L.ws[wi].nb;
-    compact += (int64_t)L.ws[wi].T * ((L.ws[wi].nb + 1) >> 1);
+    const WorkSet<NB>& W = L.ws[wi];
+    packed += (int64_t)W.T * W.nb;
+    compact += (int64_t)W.T * ((W.nb + 1) >> 1);
+    tsum += W.T;
+    if ((int64_t)W.T * W.nb > (int64_t)long_t * long_nb) {
+      long_t = W.T;
+      long_nb = W.nb;
+    }
   }
   auto bytes = [&](int64_t taps) { return (off + 2 * taps) * (int64_t)sizeof(float2) + meta_bytes; };
   auto ctas = [&](int64_t b) { return b <= kSmem3 ? 3 : b <= kSmem2 ? 2 : b <= kSmemTaps ? 1 : 0; };
@@ -1420,7 +1430,8 @@ static void layout_group(PolyLaunch<NB>& L, GroupDesc& gd, int Qt) {
   // reads bound the kernel (64 taps of 16 channels by 3 over 2^20 samples: 137
   // us packed, 122 compact; by 10: 43 and 53).
   gd.taps = ctas(bytes(packed)) > 0 ? kTapsPacked : kTapsGlobal;
-  if (!gd.win && ctas(bytes(compact)) > 0 &&
+  const bool packed_fits = gd.taps == kTapsPacked;
+  if (!gd.win && ctas(bytes(compact)) > 0 && !(keep_packed && packed_fits) &&
       (ctas(bytes(packed)) <= 1 || ctas(bytes(compact)) > ctas(bytes(packed)) ||
        (NB >= 4 && gd.nph > 1 && gd.nph <= kShortRun)))
     gd.taps = kTapsCompact;
@@ -1440,26 +1451,23 @@ static void layout_group(PolyLaunch<NB>& L, GroupDesc& gd, int Qt) {
   // two channels by 10 over 2^22 samples: 7.2 ms with a row a thread, 4.2 with
   // two; 300 taps by 6 over 2^20: 68 us and 47).
   const int ctas_sm = std::max(1, std::min(ctas(gd.smem_bytes), NB == 8 ? 2 : 3)), warps = kThreads / 32;
+  const bool pk = gd.taps == kTapsPacked;
+  auto tap = [&](int r, int64_t t, int64_t n, int64_t half) {  // of t taps, n of all channels, half of channel pairs
+    return (double)(t * (r + 3) + (pk ? n * (1 + 2 * r) : half + n * (r >= 4 ? 2 * r + 4 : 4 * r)));
+  };
   double best_time = 0;
   for (int r = NB <= 2 ? 4 : 2; r >= 1 && !gd.win; r /= 2) {
     if (Qt % (32 * r) != 0) continue;
-    int items = 0;
-    double work = 0, cost = 0;
-    for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) {
-      const int nb = L.ws[wi].nb, n = Qt / (32 * r);
-      const bool packed_taps = gd.taps == kTapsPacked;
-      const int tap = r + (packed_taps ? nb : (nb + 1) / 2) + 3 +
-                      (packed_taps ? 2 * nb * r : r >= 4 ? 2 * nb * r + 4 * nb : 4 * nb * r);
-      items += n;
-      work += (double)n * L.ws[wi].T * tap;
-      cost = std::max(cost, (double)L.ws[wi].T * tap);
-    }
-    const double time = std::max(work / 4, (items + warps - 1) / warps * cost * 3 / ctas_sm);
+    const int blocks = Qt / (32 * r), items = blocks * (gd.ws_end - gd.ws_begin);
+    const double work = blocks * tap(r, tsum, packed, compact);
+    const double round = tap(r, long_t, (int64_t)long_t * long_nb, (int64_t)long_t * ((long_nb + 1) >> 1));
+    const double time = std::max(work / 4, (items + warps - 1) / warps * round * 3 / ctas_sm);
     if (best_time == 0 || time < best_time) {
       best_time = time;
       gd.rows = r;
     }
   }
+  return packed_fits;
 }
 
 template <int NB>
@@ -1485,6 +1493,7 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
     L.nco_base[c] = R ? (uint32_t)(abs0_ % R) : 0u;
   }
   int ng = 0, nws = 0;
+  int64_t work = 0;  // complex multiply-adds
   int64_t rows_of[kMaxGroups];
   int qt_of[kMaxGroups];
   bool fixed_qt[kMaxGroups];
@@ -1520,6 +1529,7 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
         dmax = std::max(dmax, (int)delta);
         tmax = std::max(tmax, bt.T);
         rows = std::max<int64_t>(rows, (int64_t)J);
+        work += (int64_t)bt.T * W.nb * (int64_t)J;
       }
     }
     gd.ws_end = nws;
@@ -1562,10 +1572,12 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
           (int64_t)(qt_of[gi] / 2) * L.groups[gi].D >= (int64_t)L.groups[gi].tmax + L.groups[gi].delta_span)
         qt_of[gi] = std::max(32, (qt_of[gi] / 2) & ~31);
   }
-  for (int gi = 0; gi < ng; ++gi) {
+  // Chooses the tile of a group; false: it fits at no height.
+  bool packed_fits[kMaxGroups];
+  auto fit = [&](int gi, bool keep_packed) {
     GroupDesc& gd = L.groups[gi];
     const int qt0 = qt_of[gi], nsets = gd.ws_end - gd.ws_begin;
-    layout_group<NB>(L, gd, qt0);
+    packed_fits[gi] = layout_group<NB>(L, gd, qt0, keep_packed);
     // A lower tile where this one's samples leave no room for two more CTAs on
     // the SM, or one more, and a lower one does: not below one that stages as
     // much halo as rows or leaves a warp without rows (9700 taps of two
@@ -1577,22 +1589,41 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
       for (int room : {NB == 8 ? kSmem2 : kSmem3, kSmem2}) {
         for (int q = qt0 - 32; gd.smem_bytes > room; q -= 32) {
           if (q < 32 || (q < base && ((int64_t)q * gd.D < halo || nsets * q < kThreads))) {
-            layout_group<NB>(L, gd, qt0);
+            layout_group<NB>(L, gd, qt0, keep_packed);
             break;
           }
-          layout_group<NB>(L, gd, q);
+          layout_group<NB>(L, gd, q, keep_packed);
         }
         if (gd.smem_bytes <= room) break;
       }
     }
     while (gd.smem_bytes > 227 * 1024) {
-      if (gd.win || gd.Qt <= 32) return FDSP_ERR_UNSUPPORTED;
-      layout_group<NB>(L, gd, gd.Qt - 32);
+      if (gd.win || gd.Qt <= 32) return false;
+      layout_group<NB>(L, gd, gd.Qt - 32, keep_packed);
     }
     gd.ntiles = (int32_t)((rows_of[gi] + gd.Qt - 1) / gd.Qt);
-    if (!gd.win && gd.taps != kTapsPacked)
-      for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) L.ws[wi].taps = compact_of[wi];
+    return true;
+  };
+  // Groups that would gain by compact taps leave the launch of the others only
+  // for work that pays for one more (about 10 us with its tail: 64 channels
+  // over 300 k samples took 68 us in three launches, 60 in one).
+  const bool one_launch = ng > 1 && work < kSplitWork;
+  int64_t gain = 0;
+  bool others = false;
+  for (int gi = 0; gi < ng; ++gi) {
+    if (!fit(gi, one_launch)) return FDSP_ERR_UNSUPPORTED;
+    const GroupDesc& gd = L.groups[gi];
+    if (one_launch || gd.win || use_tc_for(group_of_d_[gd.D])) continue;
+    if (gd.taps == kTapsPacked) others = true;
+    if (gd.taps == kTapsCompact && packed_fits[gi])
+      for (int wi = gd.ws_begin; wi < gd.ws_end; ++wi) gain += (int64_t)L.ws[wi].T * L.ws[wi].nb * L.ws[wi].J;
   }
+  if (!one_launch && others && gain > 0 && gain < kSplitWork)
+    for (int gi = 0; gi < ng; ++gi)
+      if (L.groups[gi].taps == kTapsCompact && packed_fits[gi] && !fit(gi, true)) return FDSP_ERR_UNSUPPORTED;
+  for (int gi = 0; gi < ng; ++gi)
+    if (!L.groups[gi].win && L.groups[gi].taps != kTapsPacked)
+      for (int wi = L.groups[gi].ws_begin; wi < L.groups[gi].ws_end; ++wi) L.ws[wi].taps = compact_of[wi];
   // tensor-core groups: one prep launch and one filter-bank launch for all of
   // them; groups the tensor-core plan cannot hold stay on the FP32 kernel
   std::vector<char> on_tc(ng, 0);
@@ -1643,19 +1674,24 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
                                     reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsGlobal, false>),
                                     reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsPacked, true>),
                                     reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsGlobal, true>)};
-    const int taps_of[5] = {kTapsPacked, kTapsCompact, kTapsGlobal, kTapsPacked, kTapsGlobal};
-    for (int variant = 0; variant < 15; ++variant) {
-      const int kind = variant % 5;
-      const int size = variant / 5;  // CTAs that fit an SM: three or more, two, one
+    // (kind of kernel, and CTAs that fit an SM: three or more, two, one)
+    int variant_of[kMaxGroups];
+    uint32_t variants = 0;
+    for (int i = 0; i < nfp; ++i) {
+      const GroupDesc& gd = L.groups[order[i]];
+      const int kind = gd.win ? (gd.taps == kTapsPacked ? 3 : 4) : gd.taps == kTapsPacked ? 0 : gd.taps == kTapsCompact ? 1 : 2;
+      variant_of[i] = kind + 5 * ((gd.smem_bytes > kSmem3) + (gd.smem_bytes > kSmem2));
+      variants |= 1u << variant_of[i];
+    }
+    for (; variants != 0u; variants &= variants - 1u) {
+      const int variant = __builtin_ctz(variants);
       bool open = false;
       for (int i = 0; i < nfp; ++i) {
+        if (variant_of[i] != variant) continue;
         const GroupDesc& gd = L.groups[order[i]];
-        if (gd.taps != taps_of[kind] || (gd.win != 0) != (kind >= 3) ||
-            (gd.smem_bytes > kSmem3) + (gd.smem_bytes > kSmem2) != size)
-          continue;
         if (!open || single) {
           Batch& nb = lb[nlb++];
-          nb.kern = kernels[kind];
+          nb.kern = kernels[variant % 5];
           nb.first = nm;
           nb.count = nb.tiles = 0;
           nb.smem = 0;
