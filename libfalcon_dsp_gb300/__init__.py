@@ -379,8 +379,10 @@ class MultiRateChannelizerCuda(_Handle):
             out = [torch.empty(max(c, 1), dtype=torch.complex64, device=x.device) for c in self.out_count(n)]
         # the ctypes arrays are rebuilt when the caller's buffers change
         # (streaming loops reuse them)
-        ptrs = tuple([o.data_ptr() for o in out])
-        sizes = tuple([o.numel() for o in out])
+        try:  # (tensors; looking the methods up on each of 64 took 2 us more)
+            ptrs, sizes = tuple(map(torch.Tensor.data_ptr, out)), tuple(map(torch.Tensor.numel, out))
+        except TypeError:  # any objects with an address and a size
+            ptrs, sizes = tuple([o.data_ptr() for o in out]), tuple([o.numel() for o in out])
         oc = getattr(self, "_out_cache", None)
         if oc is None or oc[0] != ptrs or oc[1] != sizes:
             k = self.num_channels
