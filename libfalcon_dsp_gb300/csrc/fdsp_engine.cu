@@ -1772,7 +1772,11 @@ int PolyEngine::launch_nat(const float2* d_in, uint64_t n, float2* out, bool che
   L.D = (int32_t)k.down;
   L.T = batches_[0].T;
   L.H = H_;
-  // full tiles where they give every SM two, one output a thread otherwise
+  // Columns: whole periods of U, about a thread each of a CTA; a period more
+  // where that leaves fewer than six warps (U of 129 to 191 or 65 to 95: 131/100
+  // of 2^22 samples 58 us with 131 columns, 52 with 262; 150/7 662 and 629;
+  // more columns than these gain nothing).  Full tiles where they give every SM
+  // two, one output a thread otherwise.
   L.cols = (int32_t)(k.up * std::max(1u, (uint32_t)kThreads / k.up));
   if (L.cols < 192 && L.cols + (int32_t)k.up <= kNatMaxCols) L.cols += (int32_t)k.up;
   L.per = L.M >= 2LL * num_sms_ * kNatPer * L.cols ? kNatPer : 1;

@@ -1140,7 +1140,6 @@ int PolyEngine::launch_tc(const float2* d_in, uint64_t n, float2* const* out, co
     L.err = d_err_;
     L.rec_out = d_tcrec_ + li;
     L.N = (int64_t)n;
-    L.Lc = plan.Lc;
     L.xhl_n = (int64_t)sc.xhl;
     L.H = H_;
     L.G = plan.G;

@@ -155,7 +155,6 @@ struct TcLaunch {
   int* err;                          // bounded-wait failures (mapped host memory)
   TcLaunch* rec_out;                 // device copy of this record (the prep kernel writes it)
   int64_t N;                         // block samples
-  int64_t Lc;                        // samples of the time range each CTA owns
   int64_t xhl_n;                     // samples of xhl the prep writes
   int32_t H, G, nmsets, ngroups, stages, stage_bytes, nslots;
   int32_t table_off, scratch_off;    // epilogue slot table and warps' scratch in shared memory
@@ -168,7 +167,7 @@ struct TcLaunch {
   uint32_t ctotal;                   // cost of all items, below 2^31
   int32_t cost_shift;                // its unit (TcPlan::cost_shift)
   int32_t scratch_warp;              // scratch bytes of an epilogue warp: rows of runs (if any), then records
-  uint32_t pad_;
+  uint32_t pad_[3];
   TcGroup groups[kTcMaxGroups];
   TcMset ms[kTcMaxMsets];
   TcSlot slots[kTcMaxSlots];

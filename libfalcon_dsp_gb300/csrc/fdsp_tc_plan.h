@@ -128,7 +128,7 @@ struct TcPlan {
   int table_off = 0, scratch_off = 0;         // (from the 1 KB aligned start)
   int scratch_warp = 0;                       // bytes of a warp's scratch
   int G = 0;                      // grid (CTAs)
-  int64_t Lc = 0;                 // samples of the time range each CTA owns
+  int64_t Lc = 0;                 // samples a CTA has on average (the cut by input range, tc_item_range)
   int64_t items = 0;
   uint32_t ctotal = 0;            // cost of all items, each at least 1 and scaled by 2^-cost_shift
   int cost_shift = 0;
@@ -510,8 +510,8 @@ inline int tc_finish(TcPlan& p, int64_t N, int H, int num_sms) {
   p.table_off = p.stages * sb;
   p.scratch_off = p.table_off + table;
   p.smem = p.scratch_off + scratch + 1024;
-  // schedule: each CTA owns a contiguous range of input samples and runs the
-  // items of every merge set that start in it, in input order
+  // schedule: a CTA an SM at most, each running a stretch of the item list
+  // (tc_cost_bound) in input order
   int64_t umax = 0;
   for (const TcMset& m : p.ms) {
     const int64_t P = (int64_t)m.R * kTcRows * p.groups[m.group].D;
@@ -574,8 +574,8 @@ inline int tc_plan(const std::vector<TcGroupIn>& gin, int64_t N, int H, int num_
   return tc_finish(p, N, H, num_sms);
 }
 
-// Item range [first, last) of merge set m when each CTA owns an equal range of
-// input samples.
+// Item range [first, last) of merge set m were each CTA to own an equal range of
+// input samples (the kernel cuts the item list by cost instead).
 FDSP_HD inline void tc_item_range(int64_t a, int64_t P, int64_t items, int64_t Lc, int b, int G, int64_t* first,
                           int64_t* last) {
   const int64_t v0 = (int64_t)b * Lc - a, v1 = (int64_t)(b + 1) * Lc - a;
