@@ -292,6 +292,14 @@ __device__ __forceinline__ void process_block(int rows, const float2* __restrict
 // apart) read distinct bank pairs.  Real taps (no NCO shift, resampler
 // semantics) take 2 FMAs per tap instead of 4.
 constexpr int kWinRows = 7;
+// Forms of the kernel: rows; sliding window with two CTAs an SM, whose registers
+// hold complex taps or a block of real ones read ahead; sliding window of real
+// taps with three CTAs an SM and nothing read ahead.  The last is faster where
+// three fit or the phases are few (1000 taps over 2^23 samples 762 -> 696 us,
+// 8000 of one phase 6.2 -> 5.5 ms, 100 a phase at 3/2 over 2^22 108 -> 84 us);
+// with fewer CTAs and more phases reading ahead is (4095 taps by 10 over 2^24
+// samples 1.13 ms, 1.20 without).
+constexpr int kRowForm = 0, kWinTwo = 1, kWinReal = 2;
 
 // Shared memory of a CTA that leaves room for two more, or one more, on the SM.
 constexpr int kSmem3 = 75 * 1024;
@@ -340,7 +348,7 @@ __device__ __forceinline__ void win_finish(float2 acc, const ChanMeta& cm, const
   cm.out[m] = rotate_apply(er, acc, B);
 }
 
-template <bool kReal>
+template <bool kReal, bool kAhead>
 __device__ __forceinline__ void win_sums(const float2* __restrict__ xs, const float4* __restrict__ tp, int T, int D,
                                          int P, int a0, int jl0, f32x2 (&acc)[kWinRows]) {
   // packed multiply-adds in the scalar form's order: (re, re) (x, y), then
@@ -381,9 +389,9 @@ __device__ __forceinline__ void win_sums(const float2* __restrict__ xs, const fl
     int m = 0;
     for (; m + kWinRows <= nm; m += kWinRows) {
       // circular window: sample m + u + q sits in slot (u + q) % kWinRows; real
-      // taps leave the registers to read the block's taps and samples first
-      f32x2 xn[kReal ? kWinRows : 1], gn[kReal ? kWinRows : 1];
-      if constexpr (kReal) {
+      // taps leave two CTAs the registers to read the block's taps and samples first
+      f32x2 xn[kAhead ? kWinRows : 1], gn[kAhead ? kWinRows : 1];
+      if constexpr (kAhead) {
 #pragma unroll
         for (int u = 0; u < kWinRows; ++u) {
           xn[u] = xr[m + u + kWinRows - 1];
@@ -393,7 +401,7 @@ __device__ __forceinline__ void win_sums(const float2* __restrict__ xs, const fl
 #pragma unroll
       for (int u = 0; u < kWinRows; ++u) {
         f32x2 gr, gi = 0ull;
-        if constexpr (kReal) {
+        if constexpr (kAhead) {
           put((u + kWinRows - 1) % kWinRows, xn[u]);
           gr = gn[u];
         } else {
@@ -455,8 +463,8 @@ __device__ __forceinline__ void hist_sample(const float2* __restrict__ old_hist,
 // windows overlap or wrap, else (long decimations) only the groups' windows,
 // up to kMaxSegs segments of them (seg_at / seg_gap map a staged phase to its
 // place in the row).
-template <int NBMAX, int kTaps, bool kWin>
-__global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
+template <int NBMAX, int kTaps, int kForm>
+__global__ void __launch_bounds__(kThreads, kForm == kWinTwo || (kForm == kRowForm && NBMAX == 8) ? 2 : 3)
     poly_fp32_kernel(const __grid_constant__ PolyLaunch<NBMAX> L, int first, int tiles) {
   extern __shared__ __align__(16) float2 xs[];
   grid_dependency();
@@ -592,7 +600,7 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
 
-  if constexpr (kWin) {
+  if constexpr (kForm != kRowForm) {
     // single-channel work sets: items are (work set, block of kWinRows rows),
     // blocks fastest (Qt is a multiple of 32 kWinRows)
     const int nblk = Qt / kWinRows;
@@ -611,10 +619,10 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
       if (mine) {
         const int a0 = (W.delta - G.delta_min) + (G.tmax - W.T);
         const float4* tp = kTaps != kTapsGlobal ? taps_s + W.soff : W.taps;
-        if (G.real_taps)
-          win_sums<true>(xs, tp, W.T, D, P, a0, jl0, acc);
+        if (kForm == kWinReal || G.real_taps)
+          win_sums<true, kForm == kWinTwo>(xs, tp, W.T, D, P, a0, jl0, acc);
         else
-          win_sums<false>(xs, tp, W.T, D, P, a0, jl0, acc);
+          win_sums<false, false>(xs, tp, W.T, D, P, a0, jl0, acc);
       }
       float2* const out = meta_s[0].out + row0 * U;
       __syncthreads();  // every window is summed: the tile is free
@@ -638,10 +646,10 @@ __global__ void __launch_bounds__(kThreads, kWin || NBMAX == 8 ? 2 : 3)
       const int a0 = (W.delta - G.delta_min) + (G.tmax - T);
       const float4* tp = kTaps != kTapsGlobal ? taps_s + W.soff : W.taps;
       const ChanMeta* mt = meta_s + wq * NBMAX;
-      if (G.real_taps)
-        win_sums<true>(xs, tp, T, D, P, a0, jl0, acc);
+      if (kForm == kWinReal || G.real_taps)
+        win_sums<true, kForm == kWinTwo>(xs, tp, T, D, P, a0, jl0, acc);
       else
-        win_sums<false>(xs, tp, T, D, P, a0, jl0, acc);
+        win_sums<false, false>(xs, tp, T, D, P, a0, jl0, acc);
 #pragma unroll
       for (int q = 0; q < kWinRows; ++q)
         if (j0 + q < W.J)
@@ -1669,18 +1677,22 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
     }
     std::sort(order, order + nfp, [&](int a, int b) { return cost[a] != cost[b] ? cost[a] > cost[b] : a < b; });
     const bool single = !prof_ev_.empty() || (done_fn_ && tiles > 3LL * num_sms_);
-    const void* const kernels[5] = {reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsPacked, false>),
-                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsCompact, false>),
-                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsGlobal, false>),
-                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsPacked, true>),
-                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsGlobal, true>)};
+    constexpr int kKinds = 7;
+    const void* const kernels[kKinds] = {reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsPacked, kRowForm>),
+                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsCompact, kRowForm>),
+                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsGlobal, kRowForm>),
+                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsPacked, kWinTwo>),
+                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsGlobal, kWinTwo>),
+                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsPacked, kWinReal>),
+                                    reinterpret_cast<const void*>(poly_fp32_kernel<NB, kTapsGlobal, kWinReal>)};
     // (kind of kernel, and CTAs that fit an SM: three or more, two, one)
     int variant_of[kMaxGroups];
     uint32_t variants = 0;
     for (int i = 0; i < nfp; ++i) {
       const GroupDesc& gd = L.groups[order[i]];
-      const int kind = gd.win ? (gd.taps == kTapsPacked ? 3 : 4) : gd.taps == kTapsPacked ? 0 : gd.taps == kTapsCompact ? 1 : 2;
-      variant_of[i] = kind + 5 * ((gd.smem_bytes > kSmem3) + (gd.smem_bytes > kSmem2));
+      int kind = gd.taps == kTapsPacked ? 0 : gd.taps == kTapsCompact ? 1 : 2;
+      if (gd.win) kind = (gd.taps == kTapsPacked ? 3 : 4) + (gd.real_taps && (gd.smem_bytes <= kSmem3 || gd.D <= kShortRun) ? 2 : 0);
+      variant_of[i] = kind + kKinds * ((gd.smem_bytes > kSmem3) + (gd.smem_bytes > kSmem2));
       variants |= 1u << variant_of[i];
     }
     for (; variants != 0u; variants &= variants - 1u) {
@@ -1691,7 +1703,7 @@ int PolyEngine::launch(const float2* d_in, uint64_t n, float2* const* out, cudaS
         const GroupDesc& gd = L.groups[order[i]];
         if (!open || single) {
           Batch& nb = lb[nlb++];
-          nb.kern = kernels[variant % 5];
+          nb.kern = kernels[variant % kKinds];
           nb.first = nm;
           nb.count = nb.tiles = 0;
           nb.smem = 0;
